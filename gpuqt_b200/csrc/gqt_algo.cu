@@ -136,9 +136,7 @@ Op make_op(const gqt_ham* h, int nvec = 1)
   op.pot = h->pot;
   op.pot_r = h->pot_r;
   op.xx = h->xx;
-  op.emax = h->energy_max;
-  op.inv_emax = 1.0 / h->energy_max;
-  op.lib_div = !(h->energy_max >= 0x1p-100 && h->energy_max <= 0x1p100);
+  op_emax(op, h->energy_max);
   if (h->use_codes && h->n_real == 1 && h->stage_nw > 0 && h->stage_err) {
     op.stage_nw = h->stage_nw;
     op.stage_stages = h->stage_stages;

@@ -24,6 +24,7 @@
 #include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
+#include <cmath>
 #include <cstdint>
 #include <type_traits>
 
@@ -45,7 +46,11 @@ struct Op {
   const double* __restrict__ xx;
   double emax;
   double inv_emax;  // RN(1 / emax)
-  int lib_div;      // 1: emax outside [2^-100, 2^100], divide with __ddiv_rn
+  // emax = em * 2^ee with em in [1, 2), inv_em = RN(1 / em), and the span of high words
+  // the short division serves (op_emax)
+  double em, inv_em;
+  int ee;
+  unsigned div_span;
   int wpt;  // vectors per thread chosen for this launch (0: the form's default)
   // Coded operator (null code: read the ELL arrays above): entry e is row code[e] of
   // the table, giving j - i, the hopping and xx.
@@ -79,6 +84,18 @@ struct Dot {
 };
 
 // ------------------------------------------------------------------ operator entries
+// The operator's energy scale and the constants of the division by it.
+inline void op_emax(Op& op, double emax)
+{
+  op.emax = emax;
+  op.inv_emax = 1.0 / emax;
+  int e = 0;
+  op.em = 2.0 * std::frexp(emax, &e);
+  op.inv_em = 1.0 / op.em;
+  op.ee = e - 1;
+  op.div_span = emax >= 0x1p-100 && emax <= 0x1p100 ? 2u * (1800u << 20) : 0u;
+}
+
 // The coded operator's table, staged in dynamic shared memory at kernel start
 // (n_codes * 28 bytes, passed at launch as op_smem_bytes). Every kernel that reads the
 // operator is compiled once per format: C = true reads the codes and the table, C =
@@ -160,19 +177,84 @@ struct ExactArith {
   // IEEE division on the host) and q within one ulp of a/E, r = a - qE is exact and
   // RN(q + r y) = RN(a/E). q0 = RN(a y) is within 1.5 ulp; one correction makes it
   // faithful, the second rounds correctly. The exact remainders need |a| and E well
-  // inside the normal range: zero, tiny, huge or non-finite a, and an E outside
-  // [2^-100, 2^100] (op.lib_div), take the library division.
-  static __device__ __forceinline__ double scale(double a, const Op& op)
+  // inside the normal range: |a| in [2^-900, 2^900) and E in [2^-100, 2^100]
+  // (op.div_span 0 otherwise) are tested on the exponent field, as integer work. The rest
+  // takes divide_any in the step kernels (scale2): a call to the library division in
+  // their loops cost every iteration the moves of the calling convention and the
+  // constants that cannot stay in registers across it (FP64 moment sets 1-4 % slower).
+  // The evolution and current kernels (scale) call it: they live on many resident warps
+  // with few registers, and divide_any inlined made them 1-20 % slower.
+  static constexpr unsigned kDivLo = 2u * ((1023u - 900u) << 20);
+  static constexpr unsigned kDivSpan = 2u * (1800u << 20);
+  static __device__ __forceinline__ unsigned div_key(double a)
   {
-    const double m = fabs(a);
-    if (!(m >= 0x1p-900 && m <= 0x1p900) || op.lib_div)
-      return __ddiv_rn(a, op.emax);
-    const double b = op.emax, y = op.inv_emax;
+    return (unsigned)__double2hiint(a) * 2u - kDivLo;  // the sign shifts out
+  }
+  static __device__ __forceinline__ double divide(double a, double b, double y)
+  {
     double q = __dmul_rn(a, y);
     double r = __fma_rn(-q, b, a);
     q = __fma_rn(r, y, q);
     r = __fma_rn(-q, b, a);
     return __fma_rn(r, y, q);
+  }
+  // RN(a / E) for any a and E: the quotient of the significands by the sequence above,
+  // its exponent by integer arithmetic. A subnormal result is rounded once, from the
+  // 53-bit quotient and, on a tie, the sign of its exact remainder.
+  static __device__ __forceinline__ double divide_any(double a, const Op& op)
+  {
+    const unsigned long long bits = (unsigned long long)__double_as_longlong(a);
+    const unsigned long long sign = bits & 0x8000000000000000ull;
+    unsigned long long u = bits ^ sign;
+    if (u == 0 || u >= 0x7ff0000000000000ull)
+      return a;  // zeros, infinities and NaN keep their sign and kind
+    int ea = (int)(u >> 52);
+    if (ea == 0) {
+      const int up = __clzll((long long)u) - 11;
+      u <<= up;
+      ea = 1 - up;
+    }
+    const double am =
+      __longlong_as_double((long long)((u & 0x000fffffffffffffull) | 0x3ff0000000000000ull));
+    double q = __dmul_rn(am, op.inv_em);
+    q = __fma_rn(__fma_rn(-q, op.em, am), op.inv_em, q);
+    q = __fma_rn(__fma_rn(-q, op.em, am), op.inv_em, q);
+    const double r = __fma_rn(-q, op.em, am);
+    const unsigned long long uq = (unsigned long long)__double_as_longlong(q);
+    const int e = (int)(uq >> 52) + ea - 1023 - op.ee;
+    unsigned long long m = uq & 0x000fffffffffffffull;
+    if (e >= 2047) {
+      m = 0x7ff0000000000000ull;
+    } else if (e >= 1) {
+      m |= (unsigned long long)e << 52;
+    } else if (e < -53) {
+      m = 0;
+    } else {
+      const int s = 1 - e;  // bits below the subnormal grid, 1 .. 54
+      m |= 0x0010000000000000ull;
+      const unsigned long long half = 1ull << (s - 1), rest = m & (2 * half - 1);
+      m >>= s;
+      if (rest > half || (rest == half && (r > 0.0 || (r == 0.0 && (m & 1)))))
+        ++m;
+    }
+    return __longlong_as_double((long long)(m | sign));
+  }
+  static __device__ __forceinline__ double scale(double a, const Op& op)
+  {
+    if (div_key(a) >= op.div_span)
+      return __ddiv_rn(a, op.emax);
+    return divide(a, op.emax, op.inv_emax);
+  }
+  // Both parts of a complex value, with one range test.
+  static __device__ __forceinline__ void scale2(double& a, double& b, const Op& op)
+  {
+    if (max(div_key(a), div_key(b)) >= op.div_span) {
+      a = divide_any(a, op);
+      b = divide_any(b, op);
+    } else {
+      a = divide(a, op.emax, op.inv_emax);
+      b = divide(b, op.emax, op.inv_emax);
+    }
   }
   // a*c - b*d and a*d + b*c, each product and sum rounded on its own
   static __device__ __forceinline__ double cre(double a, double b, double c, double d)
@@ -196,6 +278,11 @@ struct FastArith {
   static __device__ __forceinline__ double scale(double a, const Op& op)
   {
     return a * op.inv_emax;
+  }
+  static __device__ __forceinline__ void scale2(double& a, double& b, const Op& op)
+  {
+    a *= op.inv_emax;
+    b *= op.inv_emax;
   }
   static __device__ __forceinline__ double cre(double a, double b, double c, double d)
   {
@@ -1027,8 +1114,7 @@ __global__ void __launch_bounds__(kBlock, step_min_blocks<Z, DOT, C>()) k_step(O
         hop_row_ahead<V, Z, A>(v, cur, hc, t1, op.xlo, tr, ti);
       else
         hop_row_pre<V, Z, A, C>(op, tb, i, v, cur, t1, tr, ti);
-      tr = A::scale(tr, op);
-      ti = A::scale(ti, op);
+      A::scale2(tr, ti, op);
       if constexpr (MODE == kCheb) {
         tr = A::two_x_minus(tr, s.y0.x);
         ti = A::two_x_minus(ti, s.y0.y);
@@ -1049,8 +1135,7 @@ __global__ void __launch_bounds__(kBlock, step_min_blocks<Z, DOT, C>()) k_step(O
       double tr = A::mul(p, x.x);
       double ti = A::mul(p, x.y);
       hop_row<V, Z, A, C>(op, tb, i, v, t1, tr, ti);
-      tr = A::scale(tr, op);
-      ti = A::scale(ti, op);
+      A::scale2(tr, ti, op);
       if constexpr (MODE == kCheb) {
         const double2 y0 = ld(t0 + g, op.xlo);
         tr = A::two_x_minus(tr, y0.x);
@@ -1262,13 +1347,15 @@ __global__ void __launch_bounds__(kBlock, vec_min_blocks<VT2, Z, DOT>()) k_step_
 #pragma unroll
       for (int k = 0; k < W; ++k) {
         const double2 y0 = widen(s.y0[k]);
-        r[k] = make_double2(A::two_x_minus(A::scale(tr[k], op), y0.x),
-                            A::two_x_minus(A::scale(ti[k], op), y0.y));
+        A::scale2(tr[k], ti[k], op);
+        r[k] = make_double2(A::two_x_minus(tr[k], y0.x), A::two_x_minus(ti[k], y0.y));
       }
     } else {
 #pragma unroll
-      for (int k = 0; k < W; ++k)
-        r[k] = make_double2(A::scale(tr[k], op), A::scale(ti[k], op));
+      for (int k = 0; k < W; ++k) {
+        A::scale2(tr[k], ti[k], op);
+        r[k] = make_double2(tr[k], ti[k]);
+      }
     }
     stw<W>(out + base, r, op.xlo);
     if constexpr (DOT == kDotLeft) {
@@ -1514,13 +1601,15 @@ __global__ void __launch_bounds__(kBlock, multi_min_blocks<C, Z, DOT>()) k_step_
 #pragma unroll
           for (int k = 0; k < W; ++k) {
             const double2 y0 = widen(s.y0[k]);
-            r2[k] = make_double2(A::two_x_minus(A::scale(tr[k], op), y0.x),
-                                 A::two_x_minus(A::scale(ti[k], op), y0.y));
+            A::scale2(tr[k], ti[k], op);
+            r2[k] = make_double2(A::two_x_minus(tr[k], y0.x), A::two_x_minus(ti[k], y0.y));
           }
         } else {
 #pragma unroll
-          for (int k = 0; k < W; ++k)
-            r2[k] = make_double2(A::scale(tr[k], op), A::scale(ti[k], op));
+          for (int k = 0; k < W; ++k) {
+            A::scale2(tr[k], ti[k], op);
+            r2[k] = make_double2(tr[k], ti[k]);
+          }
         }
         stw<W>(out + base, r2);
       }

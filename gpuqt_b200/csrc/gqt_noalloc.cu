@@ -227,9 +227,7 @@ extern "C" gqt_status gqt_chebyshev_step_noalloc(const gqt_ham* h, int mode, con
   op.hop = h->hop;
   op.pot = h->pot;
   op.xx = h->xx;
-  op.emax = h->energy_max;
-  op.inv_emax = 1.0 / h->energy_max;
-  op.lib_div = !(h->energy_max >= 0x1p-100 && h->energy_max <= 0x1p100);
+  op_emax(op, h->energy_max);
   const double2* a0 = mode == 1 ? (const double2*)t0->data : nullptr;
   const double2* a1 = (const double2*)t1->data;
   double2* o = (double2*)out->data;

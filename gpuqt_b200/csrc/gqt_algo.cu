@@ -9,6 +9,7 @@
 #include "gqt_algo.h"
 #include "gqt_forms.h"
 #include "gqt_internal.h"
+#include "gqt_strip.h"
 #include "gqt_wave.cuh"
 
 namespace gqt {
@@ -257,6 +258,16 @@ struct Deferred {
     return Dot{ds->partials + (size_t)(1 + used++) * stride, ds->counter, mu, 1};
   }
 
+  // The rows of `levels` consecutive moments (levels <= len), the first one's at mu.
+  gqt_status take(int levels, double2* mu, double** rows)
+  {
+    if (used + levels > len)
+      GQT_TRY(flush(true));
+    *rows = next(mu).partials;
+    used += levels - 1;
+    return GQT_OK;
+  }
+
   gqt_status flush(bool last)
   {
     if (used == 0 || (!last && used < len))
@@ -490,12 +501,50 @@ gqt_status wave_launches(const gqt_ham* h, const FormOps* f, const gqt_vec* left
   }
 }
 
+// Whether a moment loop runs in strips: the FP64 form on one vector of a plane lattice
+// (gqt_strip.cu).
+bool strip_eligible(const gqt_ham* h, const gqt_vec* right)
+{
+  return h->n_real == 1 && right->precision == GQT_FP64 && right->nvec == 1 && h->use_codes &&
+         h->strip_geo.steps > 0;
+}
+
+// Steps k = 2 .. last of a moment loop, several per launch: T_0 = t0 (read only), T_1 in
+// bufs[0]; step k's `per` sums go to mu + k * per. The launches rotate through the four
+// buffers: two hold the inputs, two take the last two vectors.
+gqt_status strip_loop(const gqt_ham* h, const Op& op, const double2* t0, const double2* left,
+                      void* const (&bufs)[4], int last, bool pair, double2* mu, DotScratch* ds)
+{
+  const int per = pair ? 2 : 1;
+  Deferred df(ds, per);
+  const double2* prev = t0;
+  const double2* cur = (const double2*)bufs[0];
+  for (int k = 2; k <= last;) {
+    const int levels = std::min(h->strip_geo.steps, last - k + 1);
+    double2* out[2];
+    int found = 0;
+    for (int b = 0; b < 4 && found < 2; ++b)
+      if (bufs[b] != (const void*)prev && bufs[b] != (const void*)cur)
+        out[found++] = (double2*)bufs[b];
+    double* rows = nullptr;
+    GQT_TRY(df.take(levels, mu + (size_t)k * per, &rows));
+    GQT_TRY(strip_steps(h, op, pair, levels, prev, cur, out[0], out[1], left, rows, df.stride,
+                        ds->counter));
+    k += levels;
+    GQT_TRY(df.flush(k > last));
+    prev = levels >= 2 ? out[0] : cur;
+    cur = out[1];
+  }
+  return GQT_OK;
+}
+
 // The launch sequence of the moment loop (src/sigma.cu:33-61) on the current stream.
 // Buffers: T_0 = right (read only), T_1 -> A, then T_m overwrites T_{m-2} in place.
 gqt_status moment_launches(const gqt_ham* h, const FormOps* f, const gqt_vec* left,
-                           const gqt_vec* right, int M, double2* mu, void* A, void* B,
+                           const gqt_vec* right, int M, double2* mu, void* const (&bufs)[4],
                            DotScratch* ds)
 {
+  void *A = bufs[0], *B = bufs[1];
   Op op = make_op(h, right->nvec);
   op.xlo = right->xlo;
   const int V = right->nvec;
@@ -530,6 +579,9 @@ gqt_status moment_launches(const gqt_ham* h, const FormOps* f, const gqt_vec* le
     return GQT_OK;
   d.mu = mu + V;
   GQT_TRY(f->step(op, kApply, nullptr, right->data, A, left->data, &d));
+  if (bufs[2])
+    return strip_loop(h, op, (const double2*)right->data, (const double2*)left->data, bufs, M - 1,
+                      false, mu, ds);
   const void* prev = right->data;  // T_{m-2}
   void* cur = A;                   // T_{m-1}
   Deferred df(ds, V);
@@ -549,8 +601,10 @@ gqt_status moment_launches(const gqt_ham* h, const FormOps* f, const gqt_vec* le
 // k_pair_moments turns them into mu (layout [m][v]). The left stream of the direct
 // loop is not read, and the recurrence runs half as many steps.
 gqt_status moment_launches_pair(const gqt_ham* h, const FormOps* f, const gqt_vec* phi, int M,
-                                double2* mu, double2* pairs, void* A, void* B, DotScratch* ds)
+                                double2* mu, double2* pairs, void* const (&bufs)[4],
+                                DotScratch* ds)
 {
+  void *A = bufs[0], *B = bufs[1];
   Op op = make_op(h, phi->nvec);
   op.xlo = phi->xlo;
   const int V = phi->nvec;
@@ -589,10 +643,12 @@ gqt_status moment_launches_pair(const gqt_ham* h, const FormOps* f, const gqt_ve
   if (K >= 1) {
     d.mu = pairs + (size_t)2 * V;
     GQT_TRY(f->step_pair(op, kApply, nullptr, phi->data, A, d));
+    if (bufs[2])
+      GQT_TRY(strip_loop(h, op, (const double2*)phi->data, nullptr, bufs, K, true, pairs, ds));
     const void* prev = phi->data;
     void* cur = A;
     Deferred df(ds, 2 * V);
-    for (int k = 2; k <= K; ++k) {
+    for (int k = 2; !bufs[2] && k <= K; ++k) {
       void* out = (prev == phi->data) ? B : (void*)prev;
       const Dot e = df.next(pairs + (size_t)k * 2 * V);
       GQT_TRY(f->step_pair(op, kCheb, prev, cur, out, e));
@@ -830,7 +886,7 @@ extern "C" gqt_status gqt_vec_segment_sum(const gqt_vec* in, int segment, int co
 
 // ------------------------------------------------------------------ moments
 static gqt_status moments_prepare(const gqt_ham* h, const gqt_vec* left, const gqt_vec* right,
-                                  int M, const FormOps** f, void** A, void** B,
+                                  int M, bool pair, const FormOps** f, void* (&bufs)[4],
                                   DotScratch** ds)
 {
   const char* w = "gqt_moments";
@@ -844,12 +900,20 @@ static gqt_status moments_prepare(const gqt_ham* h, const gqt_vec* left, const g
   Workspace& ws = *h->ws;
   if (right->precision == GQT_FP32X) {
     // the recurrence's two buffers share the inputs' arena (one residual map)
-    *A = ws_xslot(ws, 2);
-    *B = ws_xslot(ws, 3);
+    bufs[0] = ws_xslot(ws, 2);
+    bufs[1] = ws_xslot(ws, 3);
   } else {
     const size_t bytes = right->bytes;
-    GQT_TRY(ws_vector(ws, right->precision, right->nvec, bytes, 0, A));
-    GQT_TRY(ws_vector(ws, right->precision, right->nvec, bytes, 1, B));
+    GQT_TRY(ws_vector(ws, right->precision, right->nvec, bytes, 0, &bufs[0]));
+    GQT_TRY(ws_vector(ws, right->precision, right->nvec, bytes, 1, &bufs[1]));
+    // The strip loop writes its vectors beside the two it reads: two more buffers. A
+    // lattice that leaves no memory for them runs step by step.
+    if (strip_eligible(h, right) &&
+        (ws_vector(ws, right->precision, right->nvec, bytes, 2, &bufs[2]) != GQT_OK ||
+         ws_vector(ws, right->precision, right->nvec, bytes, 3, &bufs[3]) != GQT_OK)) {
+      cudaGetLastError();
+      bufs[2] = bufs[3] = nullptr;
+    }
   }
   // Block partials: [grid][R][V][4] doubles for a batch, [grid][V][4] otherwise, followed
   // by the slab of a window of deferred moments.
@@ -864,9 +928,9 @@ static gqt_status moments_run(const gqt_ham* h, const gqt_vec* left, const gqt_v
                               int M, void* mu_dev, bool pair, const char* w)
 {
   const FormOps* f;
-  void *A, *B;
+  void* bufs[4] = {nullptr, nullptr, nullptr, nullptr};
   DotScratch* ds;
-  GQT_TRY(moments_prepare(h, left, right, M, &f, &A, &B, &ds));
+  GQT_TRY(moments_prepare(h, left, right, M, pair, &f, bufs, &ds));
   if (!mu_dev)
     return fail(GQT_ERR_ARG, "%s: null output", w);
   Workspace& ws = *h->ws;
@@ -921,8 +985,8 @@ static gqt_status moments_run(const gqt_ham* h, const gqt_vec* left, const gqt_v
     gqt_status st = GQT_OK;
     if (e == cudaSuccess) {
       const uint64_t before = gqt_launch_count();
-      st = pair ? moment_launches_pair(h, f, right, M, (double2*)mu_dev, ws.pairs, A, B, ds)
-                : moment_launches(h, f, left, right, M, (double2*)mu_dev, A, B, ds);
+      st = pair ? moment_launches_pair(h, f, right, M, (double2*)mu_dev, ws.pairs, bufs, ds)
+                : moment_launches(h, f, left, right, M, (double2*)mu_dev, bufs, ds);
       // Captured launches run later, when the graph is launched.
       ws.graph_launches[key] = gqt_launch_count() - before;
       gqt_reset_launch_count();

@@ -40,6 +40,24 @@ constexpr int kBatchTileSizes[kBatchTiles] = {256, 512, 1024};
 // Select tile size `tile` (one of kBatchTileSizes) for a realisation batch.
 gqt_status batch_set_tile(gqt_ham* h, int tile);
 
+// A coded operator as a lattice of lines: every offset j - i of its table is c1 * d1 + c0
+// (mod n) with |c1| <= 1 and |c0| <= h0; site i is column i % d1 of line i / d1. d1 0: no
+// such reading of the table.
+struct StripLattice {
+  int d1 = 0, lines = 0;
+  int h0 = 0;
+};
+
+// The launch geometry of the strip loop: strips of b0 sites (cols with the halo) in segments
+// of b1 lines, `steps` Chebyshev steps per launch.
+struct StripGeo {
+  int steps = 0;  // 0: the moment loop runs step by step
+  int cols = 0;
+  int b0 = 0, b1 = 0, strips = 0;
+  int grid = 0;
+  size_t smem = 0;
+};
+
 // Temporary vectors and graph cache reused by the algorithm entry points.
 struct Workspace;
 
@@ -132,6 +150,17 @@ struct gqt_ham {
   int stage_rnw = 0;
   int stage_rwidth[8] = {};
   int* stage_rtab = nullptr;
+  // Strip moment loop of the FP64 form (gqt_strip.cu): the coded operator as a lattice of
+  // lines, whether every hopping is real and some rows are short, the distinct rows (per
+  // pattern its length and packed offsets, and its hoppings), per site its record
+  // (potential and pattern, 16 bytes), and the launch geometry.
+  gqt::StripLattice strip;
+  int strip_real = 0, strip_pad = 0;
+  int strip_patterns = 0;
+  int* strip_pat = nullptr;
+  double2* strip_hop = nullptr;
+  uint4* strip_rec = nullptr;
+  gqt::StripGeo strip_geo;
   std::unique_ptr<gqt::Workspace> ws;
   ~gqt_ham();
 };

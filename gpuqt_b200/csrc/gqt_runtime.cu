@@ -14,6 +14,7 @@
 #include "gqt_algo.h"
 #include "gqt_forms.h"
 #include "gqt_internal.h"
+#include "gqt_strip.h"
 
 namespace gqt {
 
@@ -443,6 +444,9 @@ gqt_ham::~gqt_ham()
   cudaFree(code_xx);
   cudaFree(stage_err);
   cudaFree(stage_rtab);
+  cudaFree(strip_pat);
+  cudaFree(strip_hop);
+  cudaFree(strip_rec);
 }
 
 namespace {
@@ -657,6 +661,73 @@ bool build_codes(const Packed& P, std::vector<uint8_t>& codes, std::vector<int>&
   return true;
 }
 
+// The distinct rows (length and codes) of a coded operator, at most 256, for the strip
+// moment loop; false when there are more, or its rows are not of 3, 4 or 6 entries.
+bool build_patterns(const Packed& P, const std::vector<uint8_t>& codes,
+                    const std::vector<int>& delta, const std::vector<double2>& hop,
+                    RowPatterns& rp)
+{
+  if (P.z != 3 && P.z != 4 && P.z != 6)
+    return false;
+  auto key_at = [&](long long i) {
+    uint64_t k = (uint64_t)(P.uniform ? P.z : P.nn[i]);
+    for (int m = 0; m < P.z; ++m)
+      k = k << 8 | codes[(size_t)m * P.n + i];
+    return k;
+  };
+  // each chunk of rows collects its keys; sorted, they number the patterns
+  std::vector<std::vector<uint64_t>> found(17);
+  std::atomic<bool> overflow{false};
+  parallel_rows(P.n, [&](long long lo, long long hi, int chunk) {
+    std::unordered_map<uint64_t, int> seen;
+    uint64_t last = ~0ull;
+    for (long long i = lo; i < hi && !overflow; ++i) {
+      const uint64_t k = key_at(i);
+      if (k == last)
+        continue;
+      last = k;
+      if (seen.emplace(k, 0).second && seen.size() > 256)
+        overflow = true;
+    }
+    for (const auto& kv : seen)
+      found[chunk].push_back(kv.first);
+  });
+  if (overflow)
+    return false;
+  std::vector<uint64_t> keys;
+  for (const auto& f : found)
+    keys.insert(keys.end(), f.begin(), f.end());
+  std::sort(keys.begin(), keys.end());
+  keys.erase(std::unique(keys.begin(), keys.end()), keys.end());
+  if (keys.size() > 256)
+    return false;
+  for (uint64_t k : keys) {
+    rp.len.push_back((int)(k >> (8 * P.z)));
+    for (int m = 0; m < P.z; ++m) {
+      const int c = (int)(k >> (8 * (P.z - 1 - m)) & 255);
+      rp.delta.push_back(delta[c]);
+      rp.hop.push_back(hop[c]);
+    }
+  }
+  rp.site.resize(P.n);
+  parallel_rows(P.n, [&](long long lo, long long hi, int) {
+    std::unordered_map<uint64_t, int> id;
+    for (size_t k = 0; k < keys.size(); ++k)
+      id[keys[k]] = (int)k;
+    uint64_t last = ~0ull;
+    int at = 0;
+    for (long long i = lo; i < hi; ++i) {
+      const uint64_t k = key_at(i);
+      if (k != last) {
+        last = k;
+        at = id[k];
+      }
+      rp.site[i] = (uint8_t)at;
+    }
+  });
+  return true;
+}
+
 // H = H^+ for the packed operator: for every pair of sites, the hoppings of the
 // entries i -> j summed equal the conjugate of those of j -> i (relative 1e-12).
 // Rows are short (z entries), so this is O(n z^2).
@@ -864,8 +935,12 @@ gqt_status upload_packed(const Packed& P, double energy_max, bool has_xx, gqt_ha
     h->use_codes = 1;
     if (batch_offset)
       GQT_TRY(plan_stage_windows_batch(P, codes, delta, *batch_offset, *batch_n, h));
-    else
+    else {
       plan_stage_windows(P, codes, delta, h);
+      RowPatterns rp;
+      if (build_patterns(P, codes, delta, chop, rp))
+        GQT_TRY(strip_upload(h, rp));
+    }
     GQT_CUDA(cudaMalloc(&h->stage_err, sizeof(unsigned)));
     GQT_CUDA(cudaMemset(h->stage_err, 0, sizeof(unsigned)));
   }

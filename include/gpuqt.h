@@ -140,8 +140,9 @@ gqt_status gqt_ham_set_batch_tile(gqt_ham* h, int tile_sites);
 gqt_status gqt_ham_batch_tile(const gqt_ham* h, int* tile_sites);
 
 /* The moment loop of the FP64 form (no counterpart in the reference, which launches
- * one step at a time). window 0: one launch per Chebyshev step (the default). window
- * S >= 2: the wavefront loop, S steps per persistent launch. The sites are cut into
+ * one step at a time). window 0, the default: on a plane lattice in the coded format
+ * (rows of 3, 4 or 6 entries, at most 256 distinct rows) the strip loop, 3 to 6 steps per
+ * launch, else one launch per Chebyshev step. window S >= 2: the wavefront loop, S steps per persistent launch. The sites are cut into
  * chunks; each block takes (step, chunk) items from a ticket counter in an order in
  * which every item depends only on earlier tickets, and starts one as soon as the
  * previous step is done on the chunks its rows reach. So the S steps run as a wave

@@ -126,6 +126,8 @@ Op make_op(const gqt_ham* h, int nvec = 1)
     op.code_hop = h->code_hop;
     op.code_xx = h->code_xx;
     op.n_codes = h->n_codes;
+    op.code_pack = h->code_pack;
+    op.real_hop = h->real_hop;
   }
   op.wpt = (nvec >= 0 && nvec <= 32) ? h->wpt[nvec] : 0;
   op.n = h->n;

@@ -108,6 +108,8 @@ struct gqt_ham {
   // most GQT_MAX_CODES distinct values, as lattice models do): one byte per entry and
   // a small table holding the same doubles, so results are unchanged.
   uint8_t* code = nullptr;      // [z*n] column-major
+  void* code_pack = nullptr;    // rows of 3, 4 or 6: each site's z codes, 4 or 8 bytes
+  int real_hop = 0;             // every hopping of the table is real
   int* code_delta = nullptr;    // [n_codes]: j - i
   double2* code_hop = nullptr;  // [n_codes]
   double* code_xx = nullptr;    // [n_codes]
@@ -151,11 +153,11 @@ struct gqt_ham {
   int stage_rwidth[8] = {};
   int* stage_rtab = nullptr;
   // Strip moment loop of the FP64 form (gqt_strip.cu): the coded operator as a lattice of
-  // lines, whether every hopping is real and some rows are short, the distinct rows (per
+  // lines, whether some rows are short, the distinct rows (per
   // pattern its length and packed offsets, and its hoppings), per site its record
   // (potential and pattern, 16 bytes), and the launch geometry.
   gqt::StripLattice strip;
-  int strip_real = 0, strip_pad = 0;
+  int strip_pad = 0;
   int strip_patterns = 0;
   int* strip_pat = nullptr;
   double2* strip_hop = nullptr;

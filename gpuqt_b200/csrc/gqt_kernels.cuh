@@ -55,6 +55,8 @@ struct Op {
   // Coded operator (null code: read the ELL arrays above): entry e is row code[e] of
   // the table, giving j - i, the hopping and xx.
   const uint8_t* __restrict__ code;
+  const void* __restrict__ code_pack;  // staged step: gqt_ham::code_pack
+  int real_hop;                        // every hopping of the table is real
   const int* __restrict__ code_delta;
   const double2* __restrict__ code_hop;
   const double* __restrict__ code_xx;
@@ -2007,6 +2009,22 @@ __global__ void __launch_bounds__(kBlock) k_segment_sum(const double2* __restric
       csum_merge(i, CSum{sh[w][2], sh[w][3]});
     }
     out[blockIdx.x] = make_double2(__dadd_rn(r.s, r.c), __dadd_rn(i.s, i.c));
+  }
+}
+
+// The z codes of each site in one word (z <= 4) or two, from the column-major codes.
+template <typename CodeT>
+__global__ void __launch_bounds__(kBlock) k_pack_codes(const uint8_t* __restrict__ code, int n,
+                                                       int z, CodeT* __restrict__ out)
+{
+  for (int i = blockIdx.x * kBlock + threadIdx.x; i < n; i += gridDim.x * kBlock) {
+    unsigned w[2] = {0u, 0u};
+    for (int m = 0; m < z; ++m)
+      w[m >> 2] |= (unsigned)code[(size_t)m * n + i] << (8 * (m & 3));
+    if constexpr (sizeof(CodeT) == 4)
+      out[i] = w[0];
+    else
+      out[i] = make_uint2(w[0], w[1]);
   }
 }
 

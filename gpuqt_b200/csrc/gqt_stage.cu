@@ -150,6 +150,46 @@ __device__ __forceinline__ float4 scaled_hop(double2 h, const Op& op)
   return make_float4(x.x, y.x, x.y, y.y);
 }
 
+// Two FP32 values in a register pair, and arithmetic on both at once (each rounded on its
+// own, as the scalar operations round): half the instructions of the recurrence.
+using f32x2 = unsigned long long;
+__device__ __forceinline__ f32x2 pack2(float x, float y)
+{
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %2};" : "=l"(r) : "f"(x), "f"(y));
+  return r;
+}
+__device__ __forceinline__ float2 unpack2(f32x2 a)
+{
+  float2 r;
+  asm("mov.b64 {%0, %1}, %2;" : "=f"(r.x), "=f"(r.y) : "l"(a));
+  return r;
+}
+__device__ __forceinline__ f32x2 mul2(f32x2 a, f32x2 b)
+{
+  f32x2 r;
+  asm("mul.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 add2(f32x2 a, f32x2 b)
+{
+  f32x2 r;
+  asm("add.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 sub2(f32x2 a, f32x2 b)
+{
+  f32x2 r;
+  asm("sub.rn.f32x2 %0, %1, %2;" : "=l"(r) : "l"(a), "l"(b));
+  return r;
+}
+__device__ __forceinline__ f32x2 fma2(f32x2 a, f32x2 b, f32x2 c)
+{
+  f32x2 r;
+  asm("fma.rn.f32x2 %0, %1, %2, %3;" : "=l"(r) : "l"(a), "l"(b), "l"(c));
+  return r;
+}
+
 // One vector element of the FP32 recurrence: hi and lo accumulators of both parts.
 struct AccF32 {
   float r, i, rl, il;
@@ -192,6 +232,23 @@ __device__ __forceinline__ float cheb_part(float hi, float lo, float y0)
   return __fadd_rn(s, __fmaf_rn(2.0f, lo, e));
 }
 
+// cheb_part of both parts of an element, and acc (kApply), on register pairs. The signs
+// are arranged so that no operand needs a negation: n = y0 - 2 hi = -s throughout.
+template <int MODE>
+__device__ __forceinline__ f32x2 acc_finish2(f32x2 hi, f32x2 lo, f32x2 y0)
+{
+  if constexpr (MODE == kCheb) {
+    const f32x2 two = pack2(2.0f, 2.0f), mtwo = pack2(-2.0f, -2.0f);
+    const f32x2 n = fma2(mtwo, hi, y0);
+    const f32x2 a1 = sub2(n, y0);  // -(s + y0)
+    const f32x2 b1 = sub2(n, a1);  // -(s - (s + y0))
+    const f32x2 e = add2(fma2(two, hi, a1), sub2(b1, y0));
+    return sub2(fma2(two, lo, e), n);
+  } else {
+    return add2(hi, lo);
+  }
+}
+
 // T_k = 2 acc - T_{k-2} (kCheb), or acc (kApply)
 template <int MODE>
 __device__ __forceinline__ float2 acc_finish(const AccF32& a, float2 y0)
@@ -202,13 +259,26 @@ __device__ __forceinline__ float2 acc_finish(const AccF32& a, float2 y0)
     return make_float2(a.r + a.rl, a.i + a.il);
 }
 
+// A site's z codes in one or two words (gqt_ham::code_pack).
+template <int Z>
+struct PackedCodes {
+  using type = typename std::conditional<(Z <= 4), unsigned, uint2>::type;
+};
+__device__ __forceinline__ int code_of(unsigned w, int m) { return (w >> (8 * m)) & 255; }
+__device__ __forceinline__ int code_of(uint2 w, int m)
+{
+  return ((m < 4 ? w.x : w.y) >> (8 * (m & 3))) & 255;
+}
+
 // MULTI: one step of a realisation batch (op.stage_rtab: each model's windows; md: the
 // models' tiles and the per-block, per-model sum slots that k_tile_reduce combines).
 // Tiles never straddle two models (every model is padded to 1024 sites). A block's
 // tiles come in increasing order, so the models it meets are consecutive runs: when the
 // next tile is in another model, the compute warps reduce their sums over the block
 // (a named barrier of the compute warps only) and write the block's slot of the model.
-template <int V, int Z, int MODE, int DOT, bool F32, bool MULTI = false>
+// REAL (GQT_FP32R): every hopping is real, and the products with the zero imaginary parts
+// are left out.
+template <int V, int Z, int MODE, int DOT, bool F32, bool MULTI, bool REAL>
 __global__ void __launch_bounds__(kStageThreads, 2)
   k_step_staged(Op op, StageLayout sl, const float2* t0, const float2* __restrict__ t1,
                 float2* out, const float2* __restrict__ left, Dot dot, MultiDot md)
@@ -219,19 +289,21 @@ __global__ void __launch_bounds__(kStageThreads, 2)
   constexpr int TS = kBlock / kTps;  // sites per tile
   constexpr int RB = V * (int)sizeof(float2);
   static_assert(kBlock % kTps == 0 && 32 % kTps == 0, "a site's threads share a warp");
+  using Codes = typename PackedCodes<Z>::type;
   extern __shared__ __align__(128) unsigned char stage_smem[];
   const int S = sl.stages;
   // per stage: full (the copies have landed) and empty (every compute warp has read it)
   uint64_t* full = reinterpret_cast<uint64_t*>(stage_smem + (size_t)S * sl.stage_bytes);
   uint64_t* empty = full + kMaxStages;
   double2* hop = reinterpret_cast<double2*>(empty + kMaxStages);
-  // GQT_FP32R: the hoppings divided by E_max as FP32 (hi, lo) parts
+  // GQT_FP32R: the hoppings divided by E_max as FP32 (hi, lo) parts, each twice: (hi.x,
+  // hi.x, lo.x, lo.x), then (-hi.y, hi.y, -lo.y, lo.y)
   float4* hopf = reinterpret_cast<float4*>(hop + op.n_codes);
   // per code: byte offset in a stage of site 0's neighbour row (-1: gathered from global
   // memory), and the offset j - i. MULTI: the byte offsets per model and code (coff) and
   // the offsets j - i per code (cdelta) instead.
-  int2* cinfo = reinterpret_cast<int2*>(hopf + op.n_codes);
-  int* coff = reinterpret_cast<int*>(hopf + op.n_codes);
+  int2* cinfo = reinterpret_cast<int2*>(hopf + 2 * op.n_codes);
+  int* coff = reinterpret_cast<int*>(hopf + 2 * op.n_codes);
   // MULTI: md's fields as values (lambdas then capture no kernel parameter by address)
   const int R = MULTI ? md.n_real : 1;
   const int* const tile_first = md.tile_first;
@@ -245,7 +317,9 @@ __global__ void __launch_bounds__(kStageThreads, 2)
 
   for (int c = threadIdx.x; c < op.n_codes; c += blockDim.x) {
     hop[c] = op.code_hop[c];
-    hopf[c] = scaled_hop(op.code_hop[c], op);
+    const float4 hf = scaled_hop(op.code_hop[c], op);
+    hopf[2 * c] = make_float4(hf.x, hf.x, hf.z, hf.z);
+    hopf[2 * c + 1] = make_float4(-hf.y, hf.y, -hf.w, hf.w);
     if constexpr (!MULTI) {
       const int d = op.code_delta[c];
       int o = -1;
@@ -300,9 +374,8 @@ __global__ void __launch_bounds__(kStageThreads, 2)
       ++r;
   };
 
-  // Thread 0: the copies of this block's tile j into stage j % S.
-  auto produce = [&](int j) {
-    const int s = j % S;
+  // The producer: the copies of this block's tile j into stage s.
+  auto produce = [&](int j, int s) {
     unsigned char* st = stage_smem + (size_t)s * sl.stage_bytes;
     const long long first = (long long)((int)blockIdx.x + j * G) * TS;
     const long long last = first + TS < n ? first + TS : n;
@@ -374,9 +447,13 @@ __global__ void __launch_bounds__(kStageThreads, 2)
     y[2] = make_float2(b.x, b.y);
     y[3] = make_float2(b.z, b.w);
   };
-  auto ldsf4 = [&](const unsigned char* row, float2 (&y)[W]) {
-    split4(*reinterpret_cast<const float4*>(row + ca * 16),
-           *reinterpret_cast<const float4*>(row + cb * 16), y);
+  auto lds2x = [&](const unsigned char* row, f32x2 (&y)[W]) {
+    const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(row + ca * 16);
+    const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(row + cb * 16);
+    y[0] = a.x;
+    y[1] = a.y;
+    y[2] = b.x;
+    y[3] = b.y;
   };
   constexpr int kSums = DOT == kDotPair ? 2 * W : W;
   CSum re[kSums], im[kSums];
@@ -388,12 +465,9 @@ __global__ void __launch_bounds__(kStageThreads, 2)
   // site l, loaded one tile ahead into registers: left is read only by the moment, so
   // it takes no shared memory
   // (GQT_FP32R: the potential's FP32 parts pr, made once per operator; GQT_FP32: p)
-  auto fetch = [&](int j, int (&c)[Z], double& p, float2& pr, float4& la, float4& lb) {
-    const int i = ((int)blockIdx.x + j * G) * TS + l;
+  auto fetch = [&](int i, Codes& c, double& p, float2& pr, float4& la, float4& lb) {
     if (i < n) {
-#pragma unroll
-      for (int m = 0; m < Z; ++m)
-        c[m] = op.code[(size_t)m * n + i];
+      c = reinterpret_cast<const Codes*>(op.code_pack)[i];
       if constexpr (F32)
         pr = op.pot_r[i];
       else
@@ -405,7 +479,7 @@ __global__ void __launch_bounds__(kStageThreads, 2)
       }
     }
   };
-  int cc[Z] = {};
+  Codes cc = {};
   double p = 0.0;
   float2 pr = {};
   float4 la = {}, lb = {};
@@ -416,20 +490,24 @@ __global__ void __launch_bounds__(kStageThreads, 2)
   // that runs out ends the loop of that warp (uniformly: __any_sync) or of the producer.
   const bool compute = threadIdx.x < kBlock;
   if (threadIdx.x == kBlock) {
-    int issued = 0;
+    int issued = 0, s = 0;
+    unsigned ph = 1;  // of the stage's empty barrier: its first phase ends with tile s + S
     for (int jj = 0; jj < mine; ++jj) {
-      const int s = jj % S;
       if (MULTI && *(volatile int*)&abort_flag)
         break;
-      if (jj >= S && !mbar_wait(empty + s, (unsigned)(jj / S - 1) & 1u)) {
+      if (jj >= S && !mbar_wait(empty + s, ph)) {
         atomicOr(op.stage_err, 1u);
         if constexpr (MULTI)
           *(volatile int*)&abort_flag = 1;
         break;
       }
       fence_async_smem();
-      produce(jj);
+      produce(jj, s);
       issued = jj + 1;
+      if (++s == S) {
+        s = 0;
+        ph ^= 1u;
+      }
     }
     // every copy issued has landed before the block leaves
     for (int jj = issued > S ? issued - S : 0; jj < issued; ++jj)
@@ -489,33 +567,36 @@ __global__ void __launch_bounds__(kStageThreads, 2)
       touched |= 1u << rr;
     }
   };
+  int i = (int)blockIdx.x * TS + l;  // this thread's site of the tile
+  const int step = G * TS;
+  int s = 0;         // the tile's stage, and the phase of its full barrier
+  unsigned ph = 0;
   if (compute && mine > 0) {
-    fetch(0, cc, p, pr, la, lb);
+    fetch(i, cc, p, pr, la, lb);
     if constexpr (MULTI) {
       rc = 0;
       model_of(0, rc);
     }
   }
-  for (int j = 0; compute && j < mine; ++j) {
-    int cn[Z] = {};
+  for (int j = 0; compute && j < mine; ++j, i += step) {
+    Codes cn = {};
     double pn = 0.0;
     float2 prn = {};
     float4 lan = {}, lbn = {};
     if (j + 1 < mine)
-      fetch(j + 1, cn, pn, prn, lan, lbn);
+      fetch(i + step, cn, pn, prn, lan, lbn);
     int cbase = 0;     // MULTI: the model's row of the code table
     int own = xofs;    // the site's own row in the stage
     if constexpr (MULTI) {
       cbase = rc * op.n_codes;
       own = sl.win_off[0] - rlo[rc * kStageWin] * RB;
     }
-    const int s = j % S;
     bool skip = false;
     if constexpr (MULTI) {
       // After a wait ran out (in any warp) the block skips its remaining tiles but keeps
       // taking part in the flushes, so no named barrier waits for a warp that left.
       const bool stop = *(volatile int*)&abort_flag != 0;
-      const bool late = !stop && !mbar_wait(full + s, (unsigned)(j / S) & 1u);
+      const bool late = !stop && !mbar_wait(full + s, ph);
       if (__any_sync(0xffffffffu, late)) {
         if (late)
           atomicOr(op.stage_err, 1u);
@@ -523,7 +604,7 @@ __global__ void __launch_bounds__(kStageThreads, 2)
       }
       skip = __any_sync(0xffffffffu, stop || late);
     } else {
-      const bool late = !mbar_wait(full + s, (unsigned)(j / S) & 1u);
+      const bool late = !mbar_wait(full + s, ph);
       if (__any_sync(0xffffffffu, late)) {
         if (late)
           atomicOr(op.stage_err, 1u);
@@ -531,54 +612,92 @@ __global__ void __launch_bounds__(kStageThreads, 2)
       }
     }
     const unsigned char* st = stage_smem + (size_t)s * sl.stage_bytes + l * RB;
-    const int i = ((int)blockIdx.x + j * G) * TS + l;
     if (!skip && F32 && i < n) {
-      float2 x[W];
-      ldsf4(st + own, x);
-      const float2 pf = pr;
-      AccF32 acc[W];
+      f32x2 x[W], hi[W], lo[W];
+      lds2x(st + own, x);
+      const f32x2 ph2 = pack2(pr.x, pr.x), pl2 = pack2(pr.y, pr.y);
 #pragma unroll
-      for (int k = 0; k < W; ++k)
-        acc[k] = acc_start(pf, x[k]);
+      for (int k = 0; k < W; ++k) {
+        hi[k] = mul2(ph2, x[k]);
+        lo[k] = mul2(pl2, x[k]);
+      }
+      int2 ci[Z];
+      int low = 0;  // negative where an entry lies in no window
 #pragma unroll
       for (int m = 0; m < Z; ++m) {
-        const int c = cc[m];
-        const int2 ci = MULTI ? make_int2(coff[cbase + c], cdelta[c]) : cinfo[c];
-        const float4 h = hopf[c];
-        float2 y[W];
-        if (ci.x >= 0) {
-          ldsf4(st + ci.x, y);
-        } else {
-          const float4* row = reinterpret_cast<const float4*>(t1 + (size_t)(i + ci.y) * V);
-          split4(__ldg(row + ca), __ldg(row + cb), y);
-        }
-#pragma unroll
-        for (int k = 0; k < W; ++k)
-          cmac_f32(acc[k], h, y[k]);
+        const int c = code_of(cc, m);
+        ci[m] = MULTI ? make_int2(coff[cbase + c], cdelta[c]) : cinfo[c];
+        low = min(low, ci[m].x);
       }
-      float2 y0[W] = {};
+      auto entry = [&](int m, const f32x2 (&y)[W]) {
+        const int c = code_of(cc, m);
+        const ulonglong2 h = *reinterpret_cast<const ulonglong2*>(hopf + 2 * c);
+#pragma unroll
+        for (int k = 0; k < W; ++k) {
+          hi[k] = fma2(h.x, y[k], hi[k]);
+          lo[k] = fma2(h.y, y[k], lo[k]);
+        }
+        if constexpr (!REAL) {
+          const ulonglong2 g = *reinterpret_cast<const ulonglong2*>(hopf + 2 * c + 1);
+#pragma unroll
+          for (int k = 0; k < W; ++k) {
+            const float2 t = unpack2(y[k]);
+            const f32x2 z = pack2(t.y, t.x);
+            hi[k] = fma2(g.x, z, hi[k]);
+            lo[k] = fma2(g.y, z, lo[k]);
+          }
+        }
+      };
+      if (low >= 0) {
+#pragma unroll
+        for (int m = 0; m < Z; ++m) {
+          f32x2 y[W];
+          lds2x(st + ci[m].x, y);
+          entry(m, y);
+        }
+      } else {
+#pragma unroll
+        for (int m = 0; m < Z; ++m) {
+          f32x2 y[W];
+          if (ci[m].x >= 0) {
+            lds2x(st + ci[m].x, y);
+          } else {
+            const ulonglong2* row =
+              reinterpret_cast<const ulonglong2*>(t1 + (size_t)(i + ci[m].y) * V);
+            const ulonglong2 a = __ldg(row + ca), b = __ldg(row + cb);
+            y[0] = a.x;
+            y[1] = a.y;
+            y[2] = b.x;
+            y[3] = b.y;
+          }
+          entry(m, y);
+        }
+      }
+      f32x2 y0[W] = {};
       if constexpr (MODE == kCheb)
-        ldsf4(st + sl.t0_off, y0);
-      float2 r[W];
+        lds2x(st + sl.t0_off, y0);
+      f32x2 r[W];
 #pragma unroll
       for (int k = 0; k < W; ++k)
-        r[k] = acc_finish<MODE>(acc[k], y0[k]);
-      float4* orow = reinterpret_cast<float4*>(out + (size_t)i * V);
-      orow[ca] = make_float4(r[0].x, r[0].y, r[1].x, r[1].y);
-      orow[cb] = make_float4(r[2].x, r[2].y, r[3].x, r[3].y);
+        r[k] = acc_finish2<MODE>(hi[k], lo[k], y0[k]);
+      ulonglong2* orow = reinterpret_cast<ulonglong2*>(out + (size_t)i * V);
+      orow[ca] = make_ulonglong2(r[0], r[1]);
+      orow[cb] = make_ulonglong2(r[2], r[3]);
       if constexpr (DOT == kDotLeft) {
         float2 lf[W];
         split4(la, lb, lf);
 #pragma unroll
         for (int k = 0; k < W; ++k) {
-          const double rx = r[k].x, ry = r[k].y, lx = lf[k].x, ly = lf[k].y;
+          const float2 t = unpack2(r[k]);
+          const double rx = t.x, ry = t.y, lx = lf[k].x, ly = lf[k].y;
           re[k].s = fma(rx, lx, fma(ry, ly, re[k].s));
           im[k].s = fma(ry, lx, fma(-rx, ly, im[k].s));
         }
       } else if constexpr (DOT == kDotPair) {
 #pragma unroll
         for (int k = 0; k < W; ++k) {
-          const double ox = r[k].x, oy = r[k].y, xx = x[k].x, xy = x[k].y;
+          const float2 t = unpack2(r[k]), u = unpack2(x[k]);
+          const double ox = t.x, oy = t.y, xx = u.x, xy = u.y;
           re[2 * k].s = fma(ox, ox, fma(oy, oy, re[2 * k].s));
           re[2 * k + 1].s = fma(ox, xx, fma(oy, xy, re[2 * k + 1].s));
           im[2 * k + 1].s = fma(oy, xx, fma(-ox, xy, im[2 * k + 1].s));
@@ -596,7 +715,7 @@ __global__ void __launch_bounds__(kStageThreads, 2)
       }
 #pragma unroll
       for (int m = 0; m < Z; ++m) {
-        const int c = cc[m];
+        const int c = code_of(cc, m);
         const int2 ci = MULTI ? make_int2(coff[cbase + c], cdelta[c]) : cinfo[c];
         const double2 h = hop[c];
         double2 y[W];
@@ -658,9 +777,11 @@ __global__ void __launch_bounds__(kStageThreads, 2)
     __syncwarp();
     if (!skip && (threadIdx.x & 31) == 0)
       mbar_arrive(empty + s);
-#pragma unroll
-    for (int m = 0; m < Z; ++m)
-      cc[m] = cn[m];
+    cc = cn;
+    if (++s == S) {
+      s = 0;
+      ph ^= 1u;
+    }
     p = pn;
     pr = prn;
     la = lan;
@@ -757,7 +878,7 @@ bool stage_layout(const Op& op, int V, int mode, int dot, int stages, StageLayou
 size_t stage_table_bytes(const Op& op, int R)
 {
   const size_t base = 2 * kMaxStages * sizeof(uint64_t) +
-                      (size_t)op.n_codes * (sizeof(double2) + sizeof(float4));
+                      (size_t)op.n_codes * (sizeof(double2) + 2 * sizeof(float4));
   if (R <= 1)
     return base + (size_t)op.n_codes * sizeof(int2);
   return base + ((size_t)R * op.n_codes + op.n_codes + (size_t)R * (kStageWin + 1)) * sizeof(int);
@@ -776,12 +897,12 @@ int multi_stage_budget(const Op& op, int R, int V, int dot)
   return (104 << 10) - added - kComputeWarps * kVS * 4 * (int)sizeof(double);
 }
 
-template <int V, int Z, int MODE, int DOT, bool F32, bool MULTI>
-gqt_status launch_staged(const Op& op, const StageLayout& sl, const float2* t0,
+template <int V, int Z, int MODE, int DOT, bool F32, bool MULTI, bool REAL>
+gqt_status launch_staged_as(const Op& op, const StageLayout& sl, const float2* t0,
                          const float2* t1, float2* out, const float2* left, const Dot& d,
                          MultiDot md)
 {
-  auto* kernel = k_step_staged<V, Z, MODE, DOT, F32, MULTI>;
+  auto* kernel = k_step_staged<V, Z, MODE, DOT, F32, MULTI, REAL>;
   const int R = MULTI ? md.n_real : 1;
   const size_t smem = (size_t)sl.stages * sl.stage_bytes + stage_table_bytes(op, R);
   static std::mutex mu;
@@ -818,6 +939,16 @@ gqt_status launch_staged(const Op& op, const StageLayout& sl, const float2* t0,
   count_launches(1);
   GQT_CUDA(cudaGetLastError());
   return GQT_OK;
+}
+
+template <int V, int Z, int MODE, int DOT, bool F32, bool MULTI>
+gqt_status launch_staged(const Op& op, const StageLayout& sl, const float2* t0,
+                         const float2* t1, float2* out, const float2* left, const Dot& d,
+                         const MultiDot& md)
+{
+  if (F32 && op.real_hop)
+    return launch_staged_as<V, Z, MODE, DOT, F32, MULTI, F32>(op, sl, t0, t1, out, left, d, md);
+  return launch_staged_as<V, Z, MODE, DOT, F32, MULTI, false>(op, sl, t0, t1, out, left, d, md);
 }
 
 template <int V, bool F32, bool MULTI = false>
@@ -863,7 +994,7 @@ gqt_status staged_v(const Op& op, int mode, int dot, const StageLayout& sl, cons
 static bool stage_fits(const Op& op, int nvec, int mode, int dot, bool f32, StageLayout& sl,
                        int R = 1)
 {
-  if (op.stage_nw <= 0 || !op.code || !op.stage_err || (mode != kApply && mode != kCheb))
+  if (op.stage_nw <= 0 || !op.code_pack || !op.stage_err || (mode != kApply && mode != kCheb))
     return false;
   if ((op.stage_rtab != nullptr) != (R > 1) || (R > 1 && !f32))
     return false;

@@ -558,7 +558,7 @@ StripGeo strip_geometry(const gqt_ham* h)
   static const int kShapes[][2] = {{6, 32}, {6, 64}, {4, 96}, {3, 128}};
   const int first = h->n < 20000 ? 0 : h->n < 300000 ? 1 : h->n < 1400000 ? 2 : 3;
   const int sms = device_info().sms;
-  const size_t tables = table_bytes(h->strip_patterns, h->z, h->strip_real, h->strip_pad);
+  const size_t tables = table_bytes(h->strip_patterns, h->z, h->real_hop, h->strip_pad);
   for (int k = first; k < 4; ++k) {
     StripGeo g;
     g.steps = kShapes[k][0];
@@ -596,11 +596,7 @@ gqt_status strip_upload(gqt_ham* h, const RowPatterns& rp)
   h->strip = strip_lattice(h->n, rp.delta.data(), (int)rp.delta.size(), packed.data());
   if (!h->strip.d1)
     return GQT_OK;
-  h->strip_real = 1;
   h->strip_pad = h->uniform ? 0 : 1;
-  for (const double2& t : rp.hop)
-    if (t.y != 0.0)
-      h->strip_real = 0;
   std::vector<int> pat((size_t)np * (z + 1));
   for (int k = 0; k < np; ++k) {
     pat[(size_t)k * (z + 1)] = rp.len[k];
@@ -679,8 +675,8 @@ gqt_status strip_steps(const gqt_ham* h, const Op& op, bool pair, int levels, co
     constexpr int Z = decltype(zc)::value;
     constexpr int D = decltype(dc)::value;
     if (h->strip_pad)
-      return h->strip_real ? go(k_strip<Z, D, true, true>) : go(k_strip<Z, D, false, true>);
-    return h->strip_real ? go(k_strip<Z, D, true, false>) : go(k_strip<Z, D, false, false>);
+      return h->real_hop ? go(k_strip<Z, D, true, true>) : go(k_strip<Z, D, false, true>);
+    return h->real_hop ? go(k_strip<Z, D, true, false>) : go(k_strip<Z, D, false, false>);
   };
   auto with_dot = [&](auto zc) -> gqt_status {
     return pair ? pick(zc, std::integral_constant<int, kDotPair>{})

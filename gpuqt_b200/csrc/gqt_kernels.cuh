@@ -418,12 +418,23 @@ __device__ __forceinline__ CSum shfl_xor(const CSum& a, int off)
   return b;
 }
 
+// Barrier of the block, or (SUMS, in a block that also has a copying warp) of its first
+// kBlock threads, which hold the sums.
+template <bool SUMS>
+__device__ __forceinline__ void sums_sync()
+{
+  if constexpr (SUMS)
+    asm volatile("bar.sync 1, %0;" ::"n"(kBlock) : "memory");
+  else
+    __syncthreads();
+}
+
 // The grid stage of a moment: one block combines the partials of nblocks blocks
 // ([block][V][4]) in fixed block order and writes mu[v] for v < V. Thread t sums
 // blocks t/V, t/V + kBlock/V, ... of vector t % V; lanes and warps then merge in a
 // fixed pattern, so the result depends only on nblocks and the partials. Must be
-// reached by every thread of the block.
-template <int V>
+// reached by the block's first kBlock threads, all of them when SUMS is false.
+template <int V, bool SUMS = false>
 __device__ __forceinline__ void grid_combine(const double* partials, int nblocks, double2* mu,
                                              double (&sh)[kBlock / 32][V][4])
 {
@@ -432,8 +443,7 @@ __device__ __forceinline__ void grid_combine(const double* partials, int nblocks
   const int v = threadIdx.x % V;
   constexpr int kStride = kBlock / V;
   CSum r{0.0, 0.0}, i{0.0, 0.0};
-  // threads past kBlock (a block with a producer warp) take no part
-  int b = threadIdx.x < kBlock ? (int)threadIdx.x / V : nblocks;
+  int b = (int)threadIdx.x / V;
   // Four blocks' partials are loaded before they are merged (in block order), so the
   // L2 round trips overlap.
   for (; b + 3 * kStride < nblocks; b += 4 * kStride) {
@@ -461,14 +471,14 @@ __device__ __forceinline__ void grid_combine(const double* partials, int nblocks
     csum_merge(r, shfl_xor(r, off));
     csum_merge(i, shfl_xor(i, off));
   }
-  __syncthreads();
-  if (lane < V && warp < kWarps) {
+  sums_sync<SUMS>();
+  if (lane < V) {
     sh[warp][lane][0] = r.s;
     sh[warp][lane][1] = r.c;
     sh[warp][lane][2] = i.s;
     sh[warp][lane][3] = i.c;
   }
-  __syncthreads();
+  sums_sync<SUMS>();
   if (threadIdx.x < V) {
     CSum rr{sh[0][v][0], sh[0][v][1]}, ii{sh[0][v][2], sh[0][v][3]};
     for (int w = 1; w < kWarps; ++w) {
@@ -490,15 +500,15 @@ struct ContigSlots {
 // v < V. Slot k of a thread holds the sums of vector map(q, k, W), q = lane % (V/W)
 // (by default W consecutive vectors from q W). Must be reached by every thread of the
 // block.
-// Only the first NW warps hold sums (a block may have more warps, which take no part).
-template <int V, int W, class Map = ContigSlots, int NW = kBlock / 32>
+// SUMS: the block has a further warp, which holds no sums and does not come here.
+template <int V, int W, class Map = ContigSlots, bool SUMS = false>
 __device__ __forceinline__ void dot_finish_w(CSum (&re)[W], CSum (&im)[W], const Dot& dot,
                                              Map map = Map{})
 {
   static_assert(V >= 1 && V <= 32 && (V & (V - 1)) == 0, "V must be a power of two <= 32");
   static_assert(W >= 1 && W <= V && V % W == 0, "W must divide V");
   constexpr int kTps = V / W;  // threads sharing one site
-  constexpr int kWarps = NW;
+  constexpr int kWarps = kBlock / 32;
   __shared__ double sh[kWarps][V][4];
   __shared__ unsigned is_last;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -511,7 +521,7 @@ __device__ __forceinline__ void dot_finish_w(CSum (&re)[W], CSum (&im)[W], const
       csum_merge(im[k], shfl_xor(im[k], off));
     }
   }
-  if (lane < kTps && warp < kWarps) {
+  if (lane < kTps) {
 #pragma unroll
     for (int k = 0; k < W; ++k) {
       const int v = map(lane, k, W);
@@ -521,7 +531,7 @@ __device__ __forceinline__ void dot_finish_w(CSum (&re)[W], CSum (&im)[W], const
       sh[warp][v][3] = im[k].c;
     }
   }
-  __syncthreads();
+  sums_sync<SUMS>();
   if (threadIdx.x < V) {
     const int v = threadIdx.x;
     CSum r{sh[0][v][0], sh[0][v][1]}, i{sh[0][v][2], sh[0][v][3]};
@@ -543,14 +553,14 @@ __device__ __forceinline__ void dot_finish_w(CSum (&re)[W], CSum (&im)[W], const
   }
   if (dot.defer)
     return;  // uniform: a launch parameter
-  __syncthreads();
+  sums_sync<SUMS>();
   if (threadIdx.x == 0)
     is_last = (atomicAdd(dot.counter, 1u) == gridDim.x - 1) ? 1u : 0u;
-  __syncthreads();
+  sums_sync<SUMS>();
   if (!is_last)
     return;
   __threadfence();
-  grid_combine<V>(dot.partials, (int)gridDim.x, dot.mu, sh);
+  grid_combine<V, SUMS>(dot.partials, (int)gridDim.x, dot.mu, sh);
   if (threadIdx.x == 0)
     *dot.counter = 0u;  // ready for the next launch on this stream
 }

@@ -69,27 +69,27 @@ __device__ __forceinline__ void mbar_arrive_expect(uint64_t* b, unsigned bytes)
                : "memory");
 }
 
-// One try: true once phase `parity` of b has completed; the thread may be suspended for
-// up to about 1 microsecond (the suspend-time hint) while it has not.
 __device__ __forceinline__ void mbar_arrive(uint64_t* b)
 {
   asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(sm_addr(b)) : "memory");
 }
 
+// One try: true once phase `parity` of b has completed. (No suspend-time hint: with one the
+// compiler adds a sleep of its length to the loop around the try.)
 __device__ __forceinline__ bool mbar_test(uint64_t* b, unsigned parity)
 {
   unsigned ok;
   asm volatile(
     "{\n\t.reg .pred p;\n\t"
-    "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2, %3;\n\t"
+    "mbarrier.try_wait.parity.shared::cta.b64 p, [%1], %2;\n\t"
     "selp.u32 %0, 1, 0, p;\n\t}"
     : "=r"(ok)
-    : "r"(sm_addr(b)), "r"(parity), "r"(1000u)
+    : "r"(sm_addr(b)), "r"(parity)
     : "memory");
   return ok != 0;
 }
 
-// Wait for phase `parity` of b, for at most 2^20 tries (about a second): false when it
+// Wait for phase `parity` of b, for at most 2^20 tries: false when it
 // did not complete.
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity)
 {
@@ -805,7 +805,9 @@ __global__ void __launch_bounds__(kStageThreads, 2)
         if (!((touched >> (k / (kVS * 4))) & 1u))
           slots[k] = 0.0;
     }
-  } else {
+  } else if (compute) {
+    // (the copying warp takes no part in the sums: lanes that waited for its copying lane
+    // at every shuffle held the block 10 to 25 us after its last tile)
     // Slots in the order of even sites (chunk q, then chunk q + V/4) on every thread.
     if (sw) {
 #pragma unroll
@@ -818,9 +820,9 @@ __global__ void __launch_bounds__(kStageThreads, 2)
       }
     }
     if constexpr (DOT == kDotLeft)
-      dot_finish_w<V, W, StageSlots<kHalf, 1>, kComputeWarps>(re, im, dot, {});
+      dot_finish_w<V, W, StageSlots<kHalf, 1>, true>(re, im, dot, {});
     else if constexpr (DOT == kDotPair)
-      dot_finish_w<2 * V, 2 * W, StageSlots<kHalf, 2>, kComputeWarps>(re, im, dot, {});
+      dot_finish_w<2 * V, 2 * W, StageSlots<kHalf, 2>, true>(re, im, dot, {});
   }
 }
 

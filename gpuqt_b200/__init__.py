@@ -405,7 +405,8 @@ class Hamiltonian:
 
     def set_staging(self, stages: int) -> None:
         """Staged step of the FP32 and FP32R moment loops: -1 off; 0 automatic (the
-        default: FP32R loops are staged, FP32 loops on rows of six); 1 every loop, as
+        default: FP32R loops are staged, FP32 loops on rows of six and symmetric sets
+        of vectors of 28 MiB and more); 1 every loop, as
         many shared-memory stages as fit; 2..4 every loop, that many
         (gqt_ham_set_staging)."""
         _call("gqt_ham_set_staging", self.h, int(stages))

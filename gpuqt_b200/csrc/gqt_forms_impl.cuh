@@ -280,7 +280,7 @@ struct OpImpl {
     const size_t total = (size_t)op.n * V;
     return with_z(op.z, [&](auto zc) -> gqt_status {
       constexpr int Z = decltype(zc)::value;
-      return launch_op(k_cheb2<VT2, double2, V, Z, A, C>, total, op, (const VT2*)s0,
+      return launch_op_pdl(k_cheb2<VT2, double2, V, Z, A, C>, total, op, (const VT2*)s0,
                     (const VT2*)s1, (VT2*)s2, out, bessel, label);
     });
   }
@@ -292,7 +292,7 @@ struct OpImpl {
     const size_t total = (size_t)op.n * V;
     return with_z(op.z, [&](auto zc) -> gqt_status {
       constexpr int Z = decltype(zc)::value;
-      return launch_op(k_cheb2x<VT2, double2, V, Z, A, C>, total, op, (const VT2*)s0,
+      return launch_op_pdl(k_cheb2x<VT2, double2, V, Z, A, C>, total, op, (const VT2*)s0,
                     (const VT2*)s0x, (const VT2*)s1, (const VT2*)s1x, (VT2*)s2, (VT2*)s2x,
                     out, bessel, label);
     });

@@ -1823,6 +1823,7 @@ __global__ void __launch_bounds__(kBlock) k_cheb2(Op op, const VT2* s0,
                                                   int label)
 {
   const Tables tb = load_tables<C>(op);
+  pdl_wait();
   const size_t total = (size_t)op.n * V;
   auto item = [&](size_t g, auto&& row) {
     const int i = (int)(g / V);
@@ -1865,6 +1866,7 @@ __global__ void __launch_bounds__(kBlock) k_cheb2x(Op op, const VT2* s0, const V
                                                    double bessel, int label)
 {
   const Tables tb = load_tables<C>(op);
+  pdl_wait();
   const size_t total = (size_t)op.n * V;
   auto item = [&](size_t g, auto&& row) {
     const int i = (int)(g / V);

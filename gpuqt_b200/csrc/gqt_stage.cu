@@ -1000,14 +1000,17 @@ static bool stage_fits(const Op& op, int nvec, int mode, int dot, bool f32, Stag
     return false;
   if ((op.stage_rtab != nullptr) != (R > 1) || (R > 1 && !f32))
     return false;
-  // Automatic (0), from B200 measurements with 16 vectors on graphene 2,097,152 sites
-  // (rows of 3), square 1024^2 (rows of 4) and cubic 256^3 (rows of 6): the GQT_FP32R
-  // steps are always staged (their unstaged step ran 20-60 % slower); the GQT_FP32
-  // steps on rows of 6 only (direct 11 %, pair 11 % faster there; on rows of 3 and 4
-  // the unstaged steps, at 32 warps per SM, were as fast or 10-15 % faster).
+  // Automatic (0), from B200 measurements, us per step unstaged / staged, 16 vectors. The
+  // GQT_FP32R steps are always staged (graphene 2M 271 / 172, square 300 x 290 13.5 / 11.1,
+  // cubic 100^3 195 / 99; lattices below 2 MB a vector up to 15 % slower). The GQT_FP32
+  // steps are staged on rows of 6 (cubic 62^3 38.1 / 36.8) and in symmetric sets of
+  // vectors beyond L2's reach (graphene 2M 229 / 195, square 1400^2 230 / 195, 31 MB a
+  // vector 30.3 / 29.0, 11 MB 16.4 / 16.8); their direct steps on rows of 3 and 4 ran as
+  // fast or faster unstaged (graphene 2M 200 / 225).
   if (op.stage_stages < 0)
     return false;
-  if (op.stage_stages == 0 && !f32 && op.z < 6)
+  if (op.stage_stages == 0 && !f32 && op.z < 6 &&
+      (dot != kDotPair || (size_t)op.n * nvec * sizeof(float2) < (size_t)28 << 20))
     return false;
   if (nvec != 16 && nvec != 32)
     return false;

@@ -47,25 +47,37 @@ gqt_status launch_op(K* kernel, size_t total, const Op& op, Args... args)
   return GQT_OK;
 }
 
-// launch_op with programmatic stream serialisation: the kernel may start while the
-// previous kernel in the stream finishes, and must call pdl_wait before it reads or
-// writes anything a previous kernel produces (k_step does).
+// A launch with programmatic stream serialisation (pdl): the kernel may start while the
+// previous kernel in the stream finishes, and must call pdl_wait before it reads or writes
+// anything a previous kernel produces. The steps and evolution terms are launched so: the
+// next kernel's blocks are scheduled, and have loaded their tables, when the previous
+// kernel's last blocks end. B200, 100 moments, plain / overlapped: 4 FP64 vectors on 2,400
+// sites 377 / 327 us, cubic 20^3 symmetric FP64 183 / 152, FP32 16 vectors on cubic 20^3
+// 563 / 481, FP32R 16 vectors on 1,047,040 sites 8.85 / 8.79 ms.
 template <typename... KArgs, typename... Args>
-gqt_status launch_op_pdl(void (*kernel)(Op, KArgs...), size_t total, const Op& op, Args... args)
+gqt_status launch_pdl(void (*kernel)(KArgs...), int grid, int threads, size_t smem, bool pdl,
+                      Args... args)
 {
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(grid_for((const void*)kernel, total));
-  cfg.blockDim = dim3(kBlock);
-  cfg.dynamicSmemBytes = op_smem_bytes(op);
+  cfg.gridDim = dim3(grid);
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
   cfg.stream = stream();
   cudaLaunchAttribute attr[1];
   attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
   attr[0].val.programmaticStreamSerializationAllowed = 1;
   cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  GQT_CUDA(cudaLaunchKernelEx(&cfg, kernel, op, args...));
+  cfg.numAttrs = pdl ? 1 : 0;
+  GQT_CUDA(cudaLaunchKernelEx(&cfg, kernel, args...));
   count_launches(1);
   return GQT_OK;
+}
+
+template <typename... KArgs, typename... Args>
+gqt_status launch_op_pdl(void (*kernel)(Op, KArgs...), size_t total, const Op& op, Args... args)
+{
+  return launch_pdl(kernel, grid_for((const void*)kernel, total), kBlock, op_smem_bytes(op), true,
+                    op, args...);
 }
 
 template <typename K, typename... Args>
@@ -133,14 +145,14 @@ struct OpImpl {
           const size_t items = (size_t)op.n * (V / WW);
           if (mode == kApply) {
             if (dot)
-              return launch_op(k_step_vec<VT2, V, WW, Z, A, kApply, true, C>, items, op, a0, a1, o, l,
+              return launch_op_pdl(k_step_vec<VT2, V, WW, Z, A, kApply, true, C>, items, op, a0, a1, o, l,
                             d);
-            return launch_op(k_step_vec<VT2, V, WW, Z, A, kApply, false, C>, items, op, a0, a1, o, l,
+            return launch_op_pdl(k_step_vec<VT2, V, WW, Z, A, kApply, false, C>, items, op, a0, a1, o, l,
                           d);
           }
           if (dot)
-            return launch_op(k_step_vec<VT2, V, WW, Z, A, kCheb, true, C>, items, op, a0, a1, o, l, d);
-          return launch_op(k_step_vec<VT2, V, WW, Z, A, kCheb, false, C>, items, op, a0, a1, o, l, d);
+            return launch_op_pdl(k_step_vec<VT2, V, WW, Z, A, kCheb, true, C>, items, op, a0, a1, o, l, d);
+          return launch_op_pdl(k_step_vec<VT2, V, WW, Z, A, kCheb, false, C>, items, op, a0, a1, o, l, d);
         };
         if constexpr (W2 != W) {
           if (op.wpt == W2)
@@ -153,13 +165,12 @@ struct OpImpl {
         }
         return run(std::integral_constant<int, W>{});
       }
-      // Programmatic dependent launch for the FP64 step (+1-2 % there; the FP32 step
-      // lost 7 % with it on B200).
       auto go = [&](auto* kernel) -> gqt_status {
-        if constexpr (std::is_same<VT2, double2>::value)
-          return launch_op_pdl(kernel, total, op, a0, a1, o, l, d);
-        else
-          return launch_op(kernel, total, op, a0, a1, o, l, d);
+        // (a large FP32 step streams while the next one's early blocks would take its
+        // slots: 1,047,040 sites 2 % slower with the overlap, 720,720 sites 1 % faster)
+        const bool overlap = std::is_same<VT2, double2>::value || total <= 900000;
+        return launch_pdl(kernel, grid_for((const void*)kernel, total), kBlock, op_smem_bytes(op),
+                          overlap, op, a0, a1, o, l, d);
       };
       if (mode == kApply) {
         if (dot)
@@ -190,17 +201,17 @@ struct OpImpl {
         if constexpr (V > 1) {
           const size_t items = (size_t)op.n * (V / WP);
           if (mode == kApply)
-            return launch_op(k_step_vec<VT2, V, WP, Z, A, kApply, kDotPair, C>, items, op, a0,
+            return launch_op_pdl(k_step_vec<VT2, V, WP, Z, A, kApply, kDotPair, C>, items, op, a0,
                              a1, o, (const VT2*)nullptr, d);
-          return launch_op(k_step_vec<VT2, V, WP, Z, A, kCheb, kDotPair, C>, items, op, a0, a1,
+          return launch_op_pdl(k_step_vec<VT2, V, WP, Z, A, kCheb, kDotPair, C>, items, op, a0, a1,
                            o, (const VT2*)nullptr, d);
         } else {
           const size_t total = (size_t)op.n * V;
           if (mode == kApply)
-            return launch_op(k_step<VT2, V, Z, A, kApply, kDotPair, C>, total, op, a0, a1, o,
-                             (const VT2*)nullptr, d);
-          return launch_op(k_step<VT2, V, Z, A, kCheb, kDotPair, C>, total, op, a0, a1, o,
-                           (const VT2*)nullptr, d);
+            return launch_op_pdl(k_step<VT2, V, Z, A, kApply, kDotPair, C>, total, op, a0, a1,
+                                   o, (const VT2*)nullptr, d);
+          return launch_op_pdl(k_step<VT2, V, Z, A, kCheb, kDotPair, C>, total, op, a0, a1, o,
+                                 (const VT2*)nullptr, d);
         }
       });
     }

@@ -1269,6 +1269,7 @@ __global__ void __launch_bounds__(kBlock, vec_min_blocks<VT2, Z, DOT>()) k_step_
                                                      const VT2* __restrict__ left, Dot dot)
 {
   const Tables tb = load_tables<C>(op);
+  pdl_wait();
   constexpr int kTps = V / W;
   constexpr bool kExact = std::is_same<A, ExactArith>::value;
   const size_t items = (size_t)op.n * kTps;
@@ -1405,6 +1406,7 @@ __global__ void __launch_bounds__(kBlock, vec_min_blocks<VT2, Z, DOT>()) k_step_
     if constexpr (kPre)
       cur = nxt;
   }
+  pdl_trigger();
   if constexpr (DOT == kDotLeft)
     dot_finish_w<V, W>(re, im, dot);
   else if constexpr (DOT == kDotPair)

@@ -359,6 +359,7 @@ __global__ void __launch_bounds__(kStageThreads, 2)
     fence_async_smem();
   }
   __syncthreads();
+  pdl_wait();  // the vectors are the previous launch's
 
   const int n = op.n;
   const int G = (int)gridDim.x;
@@ -797,6 +798,7 @@ __global__ void __launch_bounds__(kStageThreads, 2)
       rc = rn;
     }
   }
+  pdl_trigger();
   if constexpr (MULTI) {
     if (compute) {
       // slots of models this block never met hold zero sums
@@ -937,10 +939,8 @@ gqt_status launch_staged_as(const Op& op, const StageLayout& sl, const float2* t
     if (md.blocks_out)
       *md.blocks_out = grid;
   }
-  kernel<<<grid, kStageThreads, smem, stream()>>>(op, sl, t0, t1, out, left, d, md);
-  count_launches(1);
-  GQT_CUDA(cudaGetLastError());
-  return GQT_OK;
+  return launch_pdl(kernel, grid, kStageThreads, smem, true, op, sl, t0, t1, out,
+                    left, d, md);
 }
 
 template <int V, int Z, int MODE, int DOT, bool F32, bool MULTI>
@@ -1145,6 +1145,7 @@ __global__ void __launch_bounds__(kBlock, r_min_blocks<Z>()) k_step_r(Op op, con
   constexpr int W = 4;
   constexpr int kTps = V / W;
   const Tables tb = load_tables<C>(op);
+  pdl_wait();
   auto ld4 = [](const float2* p, float2 (&y)[W]) {
     const float4 a = *reinterpret_cast<const float4*>(p);
     const float4 b = *reinterpret_cast<const float4*>(p + 2);
@@ -1210,6 +1211,7 @@ __global__ void __launch_bounds__(kBlock, r_min_blocks<Z>()) k_step_r(Op op, con
       }
     }
   }
+  pdl_trigger();
   if constexpr (DOT == kDotLeft)
     dot_finish_w<V, W>(re, im, dot);
   else
@@ -1230,8 +1232,8 @@ gqt_status run_r(const Op& op, int mode, const void* t0, const void* t1, void* o
   return with_z(op.z, [&](auto zc) -> gqt_status {
     constexpr int Z = decltype(zc)::value;
     if (mode == kApply)
-      return launch_op(k_step_r<V, Z, kApply, DOT, C>, items, op, a0, a1, o, lf, d);
-    return launch_op(k_step_r<V, Z, kCheb, DOT, C>, items, op, a0, a1, o, lf, d);
+      return launch_op_pdl(k_step_r<V, Z, kApply, DOT, C>, items, op, a0, a1, o, lf, d);
+    return launch_op_pdl(k_step_r<V, Z, kCheb, DOT, C>, items, op, a0, a1, o, lf, d);
   });
 }
 

@@ -62,7 +62,15 @@ def entry_bytes(coded):
     return 1 if coded else 4 + 16
 
 
+# The FP64 loop on the coded operator of this lattice runs in strips, STRIP_STEPS steps
+# per launch: a launch reads T_{m-1}, T_{m-2}, left and a 16-byte record per site (potential
+# and row pattern) and writes the last two vectors.
+STRIP_STEPS = 3
+
+
 def fp64_bytes_per_site(z=Z, coded=True):
+    if coded:
+        return (5 * 16 + 16) / STRIP_STEPS
     return z * entry_bytes(coded) + 8 + 4 * 16
 
 
@@ -79,6 +87,8 @@ def fp32x_bytes_per_site_vector(V, z=Z, coded=True):
 # A step of a symmetric (doubled) moment set reads T_{k-1} and T_{k-2} and writes T_k
 # (no left stream) and yields two moments.
 def fp64_pair_bytes_per_site_step(z=Z, coded=True):
+    if coded:
+        return (4 * 16 + 16) / STRIP_STEPS
     return z * entry_bytes(coded) + 8 + 3 * 16
 
 
@@ -403,16 +413,19 @@ def run_ours(args):
         ms = max_over_ranks(t0.elapsed_time(t1), world)
         clocks = clk.summary()
         value = world * n * M * args.steps / (ms / 1e3)
-        per_launch_s = t0.elapsed_time(t1) / 1e3 / (args.steps * M)
         coded = H.format == g.FORMAT_CODED
         fmt = "coded" if coded else "ell"
-        bpl = fp64_bytes_per_site(coded=coded) * n
+        per = STRIP_STEPS if coded else 1  # Chebyshev steps per launch
+        per_launch_s = t0.elapsed_time(t1) / 1e3 / (args.steps * M) * per
+        bpl = fp64_bytes_per_site(coded=coded) * n * per
         achieved = bpl / per_launch_s / 1e9
         traffic = None
         tp = os.path.join(ROOT, "profiles", "traffic.json")
         if os.path.exists(tp):
             with open(tp) as f:
-                traffic = json.load(f).get(f"k_step_fp64_{fmt}_graphene2m_bytes_per_launch")
+                traffic = json.load(f).get(
+                    ("k_strip_fp64" if coded else "k_step_fp64_ell") +
+                    "_graphene2m_bytes_per_launch")
 
         # --- e2e: host phase vector (pinned) -> device, moments -> host, every step
         re_h = torch.from_numpy(np.ascontiguousarray(phi[0])).pin_memory()
@@ -482,7 +495,8 @@ def run_ours(args):
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak,
                              "unit": "GB/s", "frac": achieved / hbm_peak,
                              "traffic": traffic, "peak_kind": peak_kind,
-                             "kernel": f"k_step<double2,V=1,Z=3,Exact,kCheb,dot> ({fmt})",
+                             "kernel": f"k_strip<Z=3,dot> ({STRIP_STEPS} steps per launch)"
+                             if coded else "k_step<double2,V=1,Z=3,Exact,kCheb,dot> (ell)",
                              "bytes_per_launch": bpl},
                 "cpu_baseline": cpu,
                 "e2e": e2e,

@@ -662,6 +662,28 @@ bool build_codes(const Packed& P, std::vector<uint8_t>& codes, std::vector<int>&
   return true;
 }
 
+// The last few keys met, with their values: neighbouring sites alternate among the orbitals
+// of a cell.
+struct RecentKeys {
+  uint64_t key[8];
+  int val[8];
+  int used = 0, next = 0;
+  int find(uint64_t k) const
+  {
+    for (int i = 0; i < used; ++i)
+      if (key[i] == k)
+        return val[i];
+    return -1;
+  }
+  void add(uint64_t k, int v)
+  {
+    key[next] = k;
+    val[next] = v;
+    next = (next + 1) & 7;
+    used = used < 8 ? used + 1 : 8;
+  }
+};
+
 // The distinct rows (length and codes) of a coded operator, at most 256, for the strip
 // moment loop; false when there are more, or its rows are not of 3, 4 or 6 entries.
 bool build_patterns(const Packed& P, const std::vector<uint8_t>& codes,
@@ -669,6 +691,10 @@ bool build_patterns(const Packed& P, const std::vector<uint8_t>& codes,
                     RowPatterns& rp)
 {
   if (P.z != 3 && P.z != 4 && P.z != 6)
+    return false;
+  // (an operator whose offsets are not lines' needs no patterns)
+  std::vector<int> scratch(delta.size());
+  if (!strip_lattice(P.n, delta.data(), (int)delta.size(), scratch.data()).d1)
     return false;
   auto key_at = [&](long long i) {
     uint64_t k = (uint64_t)(P.uniform ? P.z : P.nn[i]);
@@ -681,12 +707,12 @@ bool build_patterns(const Packed& P, const std::vector<uint8_t>& codes,
   std::atomic<bool> overflow{false};
   parallel_rows(P.n, [&](long long lo, long long hi, int chunk) {
     std::unordered_map<uint64_t, int> seen;
-    uint64_t last = ~0ull;
+    RecentKeys recent;
     for (long long i = lo; i < hi && !overflow; ++i) {
       const uint64_t k = key_at(i);
-      if (k == last)
+      if (recent.find(k) >= 0)
         continue;
-      last = k;
+      recent.add(k, 0);
       if (seen.emplace(k, 0).second && seen.size() > 256)
         overflow = true;
     }
@@ -715,13 +741,13 @@ bool build_patterns(const Packed& P, const std::vector<uint8_t>& codes,
     std::unordered_map<uint64_t, int> id;
     for (size_t k = 0; k < keys.size(); ++k)
       id[keys[k]] = (int)k;
-    uint64_t last = ~0ull;
-    int at = 0;
+    RecentKeys recent;
     for (long long i = lo; i < hi; ++i) {
       const uint64_t k = key_at(i);
-      if (k != last) {
-        last = k;
+      int at = recent.find(k);
+      if (at < 0) {
         at = id[k];
+        recent.add(k, at);
       }
       rp.site[i] = (uint8_t)at;
     }

@@ -269,8 +269,9 @@ gqt_status gqt_vec_segment_sum(const gqt_vec* in, int segment, int count, gqt_ve
 /* Replaces find_moments_chebyshev (src/sigma.cu:33-61):
  * mu_m = <left| T_m(H/E_max) |right>, m = 0..n_moments-1, for each of the nvec
  * vectors. mu_re/mu_im are host arrays of nvec*n_moments doubles, vector-major.
- * The Chebyshev step and the moment partial sums run in one fused kernel per
- * moment; the n_moments launches are replayed from a CUDA graph. */
+ * The Chebyshev step and the moment partial sums run fused, one moment per launch or,
+ * where several steps share a launch (gqt_ham_set_loop), one per step of it; the
+ * launches are replayed from a CUDA graph. */
 gqt_status gqt_moments(const gqt_ham* h, const gqt_vec* left, const gqt_vec* right,
                        int n_moments, double* mu_re, double* mu_im);
 /* As gqt_moments, but leaves the moments on the device (mu_dev: nvec*n_moments

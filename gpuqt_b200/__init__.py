@@ -110,6 +110,7 @@ _SIGS = {
     "gqt_vec_segment_sum": (ctypes.c_int, [_vp, ctypes.c_int, ctypes.c_int, _vp]),
     "gqt_moments": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int, _dp, _dp]),
     "gqt_moments_device": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int, _vp]),
+    "gqt_moments_check": (ctypes.c_int, [_vp]),
     "gqt_moments_form": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int, ctypes.c_int, _dp, _dp]),
     "gqt_moments_device_form": (ctypes.c_int, [_vp, _vp, _vp, ctypes.c_int, ctypes.c_int, _vp]),
     "gqt_vec_convert": (ctypes.c_int, [_vp, _vp]),
@@ -588,6 +589,12 @@ def moments_device(H: Hamiltonian, left: Vector, right: Vector, n_moments: int,
     else:
         _call("gqt_moments_device_form", H.h, left.h, right.h, n_moments, precision,
               ctypes.c_void_p(mu_dev_ptr))
+
+
+def check_moments(H: Hamiltonian) -> None:
+    """Waits for the stream; raises when a wait of a moment loop on H ran out, so that the
+    sets left on the device are not valid (gqt_moments_check)."""
+    _call("gqt_moments_check", H.h)
 
 
 def evolve(H: Hamiltonian, direction: int, dt_scaled: float, state: Vector) -> None:

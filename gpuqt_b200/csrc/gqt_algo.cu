@@ -1150,6 +1150,39 @@ extern "C" gqt_status gqt_moments(const gqt_ham* h, const gqt_vec* left, const g
   return gqt_moments_form(h, left, right, M, right->precision, mu_re, mu_im);
 }
 
+// Waits for the stream and reports a bounded wait of a moment loop on h that ran out since
+// the last report (none is expected: every wait is for a copy in flight or an earlier
+// ticket). The moments of the sets issued since then are not valid.
+static gqt_status check_waits(const gqt_ham* h, const char* w)
+{
+  Workspace& ws = *h->ws;
+  cudaStream_t s = stream();
+  unsigned wave = 0, stage = 0;
+  if (ws.wave_ctl)
+    GQT_CUDA(cudaMemcpyAsync(&wave, ws.wave_ctl + 2, sizeof(wave), cudaMemcpyDeviceToHost, s));
+  if (h->stage_err)
+    GQT_CUDA(cudaMemcpyAsync(&stage, h->stage_err, sizeof(stage), cudaMemcpyDeviceToHost, s));
+  GQT_CUDA(cudaStreamSynchronize(s));
+  if (!wave && !stage)
+    return GQT_OK;
+  if (wave)
+    GQT_CUDA(cudaMemsetAsync(ws.wave_ctl + 2, 0, sizeof(wave), s));
+  if (stage)
+    GQT_CUDA(cudaMemsetAsync(h->stage_err, 0, sizeof(stage), s));
+  GQT_CUDA(cudaStreamSynchronize(s));
+  return fail(GQT_ERR_STATE, "%s: a wait of the %s timed out; moments invalid", w,
+              wave                     ? "wavefront loop"
+              : (stage & kStripWait)   ? "strip loop"
+                                       : "staged step");
+}
+
+extern "C" gqt_status gqt_moments_check(const gqt_ham* h)
+{
+  if (!h)
+    return fail(GQT_ERR_ARG, "gqt_moments_check: null Hamiltonian");
+  return check_waits(h, "gqt_moments_check");
+}
+
 // A moment loop into the workspace's device buffer, then to host arrays [vector][m].
 static gqt_status moments_host(const gqt_ham* h, const gqt_vec* left, const gqt_vec* right,
                                int M, int precision, bool pair, double* mu_re, double* mu_im,
@@ -1191,26 +1224,7 @@ static gqt_status moments_host(const gqt_ham* h, const gqt_vec* left, const gqt_
   const double2* host = ws.mu_host;
   GQT_CUDA(cudaMemcpyAsync(ws.mu_host, ws.mu, need, cudaMemcpyDeviceToHost, stream()));
   GQT_CUDA(cudaStreamSynchronize(stream()));
-  if (ws.wave_ctl) {
-    // a wavefront loop whose bounded wait ran out flagged it (never expected: every
-    // wait is on an earlier ticket)
-    unsigned err = 0;
-    GQT_CUDA(cudaMemcpy(&err, ws.wave_ctl + 2, sizeof(unsigned), cudaMemcpyDeviceToHost));
-    if (err) {
-      GQT_CUDA(cudaMemset(ws.wave_ctl + 2, 0, sizeof(unsigned)));
-      return fail(GQT_ERR_STATE, "%s: a wait of the wavefront loop timed out; moments invalid",
-                  w);
-    }
-  }
-  if (h->stage_err) {
-    // a staged step whose bounded wait for its shared-memory copies ran out flagged it
-    unsigned err = 0;
-    GQT_CUDA(cudaMemcpy(&err, h->stage_err, sizeof(unsigned), cudaMemcpyDeviceToHost));
-    if (err) {
-      GQT_CUDA(cudaMemset(h->stage_err, 0, sizeof(unsigned)));
-      return fail(GQT_ERR_STATE, "%s: a wait of the staged step timed out; moments invalid", w);
-    }
-  }
+  GQT_TRY(check_waits(h, w));
   for (int k = 0; k < V; ++k)
     for (int m = 0; m < M; ++m) {
       mu_re[(size_t)k * M + m] = host[(size_t)m * V + k].x;

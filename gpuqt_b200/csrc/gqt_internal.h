@@ -58,6 +58,9 @@ struct StripGeo {
   size_t smem = 0;
 };
 
+// Bits of gqt_ham::stage_err: the loop whose bounded wait for its copies ran out.
+constexpr unsigned kStageWait = 1u, kStripWait = 2u;
+
 // Temporary vectors and graph cache reused by the algorithm entry points.
 struct Workspace;
 

@@ -89,11 +89,13 @@ __device__ __forceinline__ bool mbar_test(uint64_t* b, unsigned parity)
   return ok != 0;
 }
 
-// Wait for phase `parity` of b, for at most 2^20 tries: false when it
-// did not complete.
+// Wait for phase `parity` of b, for at most kMaxTries tries of about 4 us each (B200, a
+// phase that does not complete; with or without the hint), about a second: false when it did
+// not complete.
+constexpr int kMaxTries = 1 << 18;
 __device__ __forceinline__ bool mbar_wait(uint64_t* b, unsigned parity)
 {
-  for (int it = 0; it < (1 << 20); ++it)
+  for (int it = 0; it < kMaxTries; ++it)
     if (mbar_test(b, parity))
       return true;
   return false;
@@ -497,7 +499,7 @@ __global__ void __launch_bounds__(kStageThreads, 2)
       if (MULTI && *(volatile int*)&abort_flag)
         break;
       if (jj >= S && !mbar_wait(empty + s, ph)) {
-        atomicOr(op.stage_err, 1u);
+        atomicOr(op.stage_err, kStageWait);
         if constexpr (MULTI)
           *(volatile int*)&abort_flag = 1;
         break;
@@ -600,7 +602,7 @@ __global__ void __launch_bounds__(kStageThreads, 2)
       const bool late = !stop && !mbar_wait(full + s, ph);
       if (__any_sync(0xffffffffu, late)) {
         if (late)
-          atomicOr(op.stage_err, 1u);
+          atomicOr(op.stage_err, kStageWait);
         *(volatile int*)&abort_flag = 1;
       }
       skip = __any_sync(0xffffffffu, stop || late);
@@ -608,7 +610,7 @@ __global__ void __launch_bounds__(kStageThreads, 2)
       const bool late = !mbar_wait(full + s, ph);
       if (__any_sync(0xffffffffu, late)) {
         if (late)
-          atomicOr(op.stage_err, 1u);
+          atomicOr(op.stage_err, kStageWait);
         break;
       }
     }

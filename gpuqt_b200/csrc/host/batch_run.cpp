@@ -54,6 +54,7 @@ struct Group {
             "find_moments_chebyshev");
     std::vector<real> re((size_t)M * V), im((size_t)M * V);
     mu.copy_to_host(re.data(), im.data());
+    check(gqt_moments_check(H.handle()), "find_moments_chebyshev");
     for (int v = 0; v < V; ++v) {
       std::vector<real> r(M), i(M);
       for (int m = 0; m < M; ++m) {

@@ -20,20 +20,23 @@ using gqt_host::check;
 void find_moments_chebyshev(Model& model, Hamiltonian& H, Vector& state_left,
                             Vector& state_right, Vector& output)
 {
-  // One fused step+moment kernel per moment, replayed as a CUDA graph, in the form
+  // Fused step and moment kernels, replayed as a CUDA graph, in the form
   // Vector::moment_precision; the moments land in `output` (FP64, number_of_moments
-  // entries) on the device.
-  if (model.kpm_doubling && &state_left == &state_right) {
+  // entries) on the device. The set is complete and checked on return: a loop whose wait
+  // ran out ends the run here, not as wrong rows of the .out files (the drivers copy the
+  // moments to the host next, so they wait for the set either way).
+  const int M = model.number_of_moments;
+  const char* w = "find_moments_chebyshev";
+  if (model.kpm_doubling && &state_left == &state_right)
     // A symmetric set from half the steps (para.in kpm_doubling).
-    check(gqt_moments_doubled_device(H.handle(), state_right.handle(), model.number_of_moments,
+    check(gqt_moments_doubled_device(H.handle(), state_right.handle(), M,
                                      Vector::moment_precision, gqt_vec_data(output.handle())),
-          "find_moments_chebyshev");
-    return;
-  }
-  check(gqt_moments_device_form(H.handle(), state_left.handle(), state_right.handle(),
-                                model.number_of_moments, Vector::moment_precision,
-                                gqt_vec_data(output.handle())),
-        "find_moments_chebyshev");
+          w);
+  else
+    check(gqt_moments_device_form(H.handle(), state_left.handle(), state_right.handle(), M,
+                                  Vector::moment_precision, gqt_vec_data(output.handle())),
+          w);
+  check(gqt_moments_check(H.handle()), w);
 }
 
 void apply_damping(Model& model, real* re, real* im)

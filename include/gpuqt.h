@@ -276,7 +276,9 @@ gqt_status gqt_moments(const gqt_ham* h, const gqt_vec* left, const gqt_vec* rig
                        int n_moments, double* mu_re, double* mu_im);
 /* As gqt_moments, but leaves the moments on the device (mu_dev: nvec*n_moments
  * double2 (re, im), moment-major [m*nvec + k]; for a realisation batch
- * [m][r][k], n_moments*count*nvec entries) and does not synchronise. */
+ * [m][r][k], n_moments*count*nvec entries) and does not synchronise. Some loops wait on
+ * the device for their own copies, each wait with a limit: gqt_moments_check tells
+ * whether one ran out. */
 gqt_status gqt_moments_device(const gqt_ham* h, const gqt_vec* left, const gqt_vec* right,
                               int n_moments, void* mu_dev);
 /* As gqt_moments / gqt_moments_device, with the Chebyshev recurrence run in the
@@ -289,6 +291,11 @@ gqt_status gqt_moments_form(const gqt_ham* h, const gqt_vec* left, const gqt_vec
 gqt_status gqt_moments_device_form(const gqt_ham* h, const gqt_vec* left,
                                    const gqt_vec* right, int n_moments, int precision,
                                    void* mu_dev);
+/* For sets left on the device: waits for the calling thread's stream and returns
+ * GQT_ERR_STATE, once, when a wait of a moment loop on h ran out since the last report (by
+ * this call or by an entry that returns moments to the host); the sets issued since then
+ * are not valid. None is expected. No counterpart in the reference. */
+gqt_status gqt_moments_check(const gqt_ham* h);
 /* The symmetric moment set mu_m = <phi|T_m(H~)|phi>, m < n_moments, from n_moments / 2
  * Chebyshev steps, by T_j T_k = (T_{j+k} + T_{|j-k|}) / 2 (KPM "doubling": each step
  * fuses <T_k|T_k> and <T_{k-1}|T_k>; mu_2k = 2 <T_k|T_k> - mu_0, mu_{2k-1} =

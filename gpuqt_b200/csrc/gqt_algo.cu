@@ -40,6 +40,15 @@ Workspace::~Workspace()
 
 Workspace* new_workspace() { return new Workspace(); }
 
+// Device words that are zero for every stream from here on.
+static cudaError_t alloc_zeroed(unsigned** p, int count)
+{
+  cudaError_t e = cudaMalloc(p, count * sizeof(unsigned));
+  if (e == cudaSuccess)
+    e = cudaMemsetAsync(*p, 0, count * sizeof(unsigned), stream());
+  return e == cudaSuccess ? cudaStreamSynchronize(stream()) : e;
+}
+
 gqt_status ws_vector(Workspace& ws, int precision, int nvec, size_t bytes, int i, void** out)
 {
   auto& b = ws.bufs[{precision, nvec}];
@@ -75,8 +84,7 @@ gqt_status ws_dot(Workspace& ws, size_t doubles, DotScratch** out)
     ws.dot.blocks = (int)need;  // capacity in doubles
   }
   if (!ws.dot.counter) {
-    GQT_CUDA(cudaMalloc(&ws.dot.counter, 2 * sizeof(unsigned)));
-    GQT_CUDA(cudaMemset(ws.dot.counter, 0, 2 * sizeof(unsigned)));
+    GQT_CUDA(alloc_zeroed(&ws.dot.counter, 2));
   }
   *out = &ws.dot;
   return GQT_OK;
@@ -432,8 +440,7 @@ gqt_status wave_prepare(const gqt_ham* h, Workspace& ws)
     ws.wave_done_n = h->wave_chunks;
   }
   if (!ws.wave_ctl) {
-    GQT_CUDA(cudaMalloc(&ws.wave_ctl, 4 * sizeof(unsigned)));
-    GQT_CUDA(cudaMemset(ws.wave_ctl, 0, 4 * sizeof(unsigned)));
+    GQT_CUDA(alloc_zeroed(&ws.wave_ctl, 4));
   }
   return GQT_OK;
 }
@@ -815,8 +822,7 @@ extern "C" gqt_status gqt_inner_product(const gqt_vec* state, const gqt_vec* lef
   double2*& mu = t_mu[dev];
   if (!ds.partials) {
     GQT_CUDA(cudaMalloc(&ds.partials, (size_t)max_grid() * 32 * 4 * sizeof(double)));
-    GQT_CUDA(cudaMalloc(&ds.counter, sizeof(unsigned)));
-    GQT_CUDA(cudaMemset(ds.counter, 0, sizeof(unsigned)));
+    GQT_CUDA(alloc_zeroed(&ds.counter, 1));
     GQT_CUDA(cudaMalloc(&mu, 32 * sizeof(double2)));
   }
   Dot d{ds.partials, ds.counter, mu};
@@ -840,8 +846,7 @@ static DotScratch* thread_dot()
   if (!ds.partials) {
     if (cudaMalloc(&ds.partials, (size_t)max_grid() * 32 * 4 * sizeof(double)) != cudaSuccess)
       return nullptr;
-    if (cudaMalloc(&ds.counter, sizeof(unsigned)) != cudaSuccess ||
-        cudaMemset(ds.counter, 0, sizeof(unsigned)) != cudaSuccess)
+    if (alloc_zeroed(&ds.counter, 1) != cudaSuccess)
       return nullptr;
   }
   return &ds;

@@ -918,6 +918,16 @@ gqt_status plan_stage_windows_batch(const Packed& P, const std::vector<uint8_t>&
   return GQT_OK;
 }
 
+// The uploads so far are on the device. A cudaMemcpy from pageable memory may return when
+// its bytes have been staged, and it runs on the legacy stream, with which a caller's
+// non-blocking stream is not ordered: without this a kernel on such a stream could read what
+// was there before.
+gqt_status uploads_done()
+{
+  GQT_CUDA(cudaStreamSynchronize(cudaStreamLegacy));
+  return GQT_OK;
+}
+
 // batch_offset / batch_n: the models of a realisation batch (their staging windows are
 // planned per model), or null for one model.
 gqt_status upload_packed(const Packed& P, double energy_max, bool has_xx, gqt_ham* h,
@@ -968,6 +978,7 @@ gqt_status upload_packed(const Packed& P, double energy_max, bool has_xx, gqt_ha
       const size_t word = P.z <= 4 ? sizeof(unsigned) : sizeof(uint2);
       GQT_CUDA(cudaMalloc(&h->code_pack, (size_t)P.n * word));
       const int grid = std::min((P.n + kBlock - 1) / kBlock, max_grid());
+      GQT_TRY(uploads_done());
       if (P.z <= 4)
         k_pack_codes<<<grid, kBlock, 0, stream()>>>(h->code, P.n, P.z, (unsigned*)h->code_pack);
       else
@@ -1010,6 +1021,7 @@ extern "C" gqt_status gqt_ham_create(const gqt_ell_desc* d, gqt_ham** out)
     return fail(GQT_ERR_ALLOC, "gqt_ham_create: host allocation failed");
   std::unique_ptr<gqt_ham> guard(h);
   GQT_TRY(upload_packed(P, d->energy_max, d->xx != nullptr, h));
+  GQT_TRY(uploads_done());
   h->real_offset = {0, d->n};
   h->real_n = {d->n};
   h->real_emax = {d->energy_max};
@@ -1069,6 +1081,7 @@ extern "C" gqt_status gqt_ham_create_batch(const gqt_ell_desc* descs, int count,
   GQT_CUDA(cudaMalloc(&h->tile_first_all, first.size() * sizeof(int)));
   GQT_CUDA(cudaMemcpy(h->tile_first_all, first.data(), first.size() * sizeof(int),
                       cudaMemcpyHostToDevice));
+  GQT_TRY(uploads_done());
   GQT_TRY(batch_set_tile(h, kBatchTileSizes[0]));
   *out = guard.release();
   return GQT_OK;

@@ -622,6 +622,9 @@ gqt_status strip_upload(gqt_ham* h, const RowPatterns& rp)
     return GQT_OK;
   }
   cudaError_t e = cudaMemcpy(pid, rp.site.data(), (size_t)h->n, cudaMemcpyHostToDevice);
+  // (pageable memory, legacy stream: the copies may still be on their way)
+  if (e == cudaSuccess)
+    e = cudaStreamSynchronize(cudaStreamLegacy);
   if (e == cudaSuccess) {
     const int grid = std::min((h->n + kBlock - 1) / kBlock, max_grid());
     k_strip_rec<<<grid, kBlock, 0, stream()>>>(h->pot, pid, h->n, h->strip_rec);

@@ -40,3 +40,34 @@ def test_pinned_upload_then_repeated_downloads():
         got_re, got_im = v.download()
         np.testing.assert_array_equal(got_re, re.numpy())
         np.testing.assert_array_equal(got_im, im.numpy())
+
+
+def test_operator_uploaded_on_a_non_blocking_stream():
+    """The kernels that prepare an operator run on the caller's stream, which is not ordered
+    with the legacy stream of the uploads: the operator equals one uploaded on the legacy
+    stream. (The ordering itself is by the wait between them; an early kernel would show here
+    only by chance.)"""
+    import torch
+
+    from test_gpu_strip import SQUARE, lattice
+
+    ell = lattice(SQUARE, 700, 601, seed=3)
+    rng = np.random.default_rng(0)
+    ph = rng.uniform(0, 2 * np.pi, (16, ell["n"]))
+
+    def sets():
+        H = g.Hamiltonian(**ell)
+        x = g.Vector.from_host(np.cos(ph[0]), np.sin(ph[0]))
+        X = g.Vector.from_host(np.cos(ph), np.sin(ph), nvec=16, precision=g.FP32)
+        return (*g.moments(H, x, x, 12), *g.moments(H, X, X, 12, precision=g.FP32R))
+
+    want = sets()
+    side = torch.cuda.Stream()
+    try:
+        g.set_stream(side.cuda_stream)
+        for _ in range(4):
+            for got, w in zip(sets(), want):
+                np.testing.assert_array_equal(got, w)
+    finally:
+        g.sync()
+        g.set_stream(None)

@@ -95,6 +95,10 @@ inline void op_emax(Op& op, double emax)
   op.em = 2.0 * std::frexp(emax, &e);
   op.inv_em = 1.0 / op.em;
   op.ee = e - 1;
+  if (std::isinf(emax)) {  // a / inf: an exponent that takes every finite quotient to zero
+    op.em = op.inv_em = 1.0;
+    op.ee = 4096;
+  }
   op.div_span = emax >= 0x1p-100 && emax <= 0x1p100 ? 2u * (1800u << 20) : 0u;
 }
 
@@ -208,8 +212,10 @@ struct ExactArith {
     const unsigned long long bits = (unsigned long long)__double_as_longlong(a);
     const unsigned long long sign = bits & 0x8000000000000000ull;
     unsigned long long u = bits ^ sign;
-    if (u == 0 || u >= 0x7ff0000000000000ull)
-      return a;  // zeros, infinities and NaN keep their sign and kind
+    if (u == 0)
+      return a;
+    if (u >= 0x7ff0000000000000ull)
+      return __dmul_rn(a, op.inv_emax);  // inf, NaN; inf / inf is NaN (inv_emax 0)
     int ea = (int)(u >> 52);
     if (ea == 0) {
       const int up = __clzll((long long)u) - 11;

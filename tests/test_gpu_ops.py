@@ -188,3 +188,47 @@ def test_division_by_energy_max_correctly_rounded(emax):
         want = a / emax
     np.testing.assert_array_equal(re, want)
     assert np.array_equal(np.signbit(re), np.signbit(want))
+
+
+@pytest.mark.parametrize("emax", [np.inf, 1.7e308, 5e-324, 3e-310, 2.0 ** 101])
+def test_division_by_an_extreme_energy_max(emax):
+    """As above at the ends of the range of E_max: infinite (every finite quotient is a zero
+    of a's sign, inf / inf is NaN), near overflow, subnormal."""
+    rng = np.random.default_rng(7)
+    n = 1 << 14
+    a = rng.uniform(1.0, 2.0, n) * np.exp2(rng.integers(-1074, 1024, n).astype(np.float64))
+    a *= np.where(rng.random(n) < 0.5, -1.0, 1.0)
+    a[:6] = [0.0, -0.0, np.inf, -np.inf, np.nan, 5e-324]
+    H = g.Hamiltonian(n=n, max_neighbor=1, energy_max=emax,
+                      neighbor_number=np.zeros(n, np.int32),
+                      neighbor_list=np.arange(n, dtype=np.int32), potential=a,
+                      hopping_real=np.zeros(n), hopping_imag=np.zeros(n))
+    x = g.Vector.from_host(np.ones(n), np.zeros(n))
+    y = g.Vector(n)
+    g.apply(H, x, y)
+    re, _ = y.download()
+    with np.errstate(all="ignore"):
+        want = a / emax
+    np.testing.assert_array_equal(re, want)
+    number = ~np.isnan(want)
+    assert np.array_equal(np.signbit(re[number]), np.signbit(want[number]))
+
+
+def test_moments_with_an_infinite_energy_max():
+    """H / E_max = 0: T_2k = (-1)^k, T_2k+1 = 0, in the strip loop (a plane lattice of rows of
+    four) and the step loop."""
+    n0, n1 = 12, 14
+    n = n0 * n1
+    i = np.arange(n)
+    x, y = i // n1, i % n1
+    nl = np.stack([((x + 1) % n0) * n1 + y, ((x - 1) % n0) * n1 + y,
+                   x * n1 + (y + 1) % n1, x * n1 + (y - 1) % n1], 1)
+    H = g.Hamiltonian(n=n, max_neighbor=4, energy_max=np.inf, neighbor_number=np.full(n, 4),
+                      neighbor_list=nl.reshape(-1), potential=np.linspace(-1, 1, n),
+                      hopping_real=np.full(4 * n, -1.0), hopping_imag=np.zeros(4 * n))
+    phi = g.Vector.from_host(np.ones(n), np.zeros(n))
+    for fmt in (g.FORMAT_CODED, g.FORMAT_ELL):
+        H.set_format(fmt)
+        re, im = g.moments(H, phi, phi, 9)
+        np.testing.assert_array_equal(re, n * np.array([1, 0, -1, 0, 1, 0, -1, 0, 1.0]))
+        np.testing.assert_array_equal(im, np.zeros(9))

@@ -512,10 +512,10 @@ gqt_status wave_launches(const gqt_ham* h, const FormOps* f, const gqt_vec* left
 
 // Whether a moment loop runs in strips: the FP64 form on one vector of a plane lattice
 // (gqt_strip.cu).
-bool strip_eligible(const gqt_ham* h, const gqt_vec* right)
+bool strip_eligible(const gqt_ham* h, const gqt_vec* right, bool pair)
 {
   return h->n_real == 1 && right->precision == GQT_FP64 && right->nvec == 1 && h->use_codes &&
-         h->strip_geo.steps > 0;
+         h->strip_geo.steps > 0 && (h->strip_loops >> pair & 1);
 }
 
 // Steps k = 2 .. last of a moment loop, several per launch: T_0 = t0 (read only), T_1 in
@@ -915,7 +915,7 @@ static gqt_status moments_prepare(const gqt_ham* h, const gqt_vec* left, const g
     GQT_TRY(ws_vector(ws, right->precision, right->nvec, bytes, 1, &bufs[1]));
     // The strip loop writes its vectors beside the two it reads: two more buffers. A
     // lattice that leaves no memory for them runs step by step.
-    if (strip_eligible(h, right) &&
+    if (strip_eligible(h, right, pair) &&
         (ws_vector(ws, right->precision, right->nvec, bytes, 2, &bufs[2]) != GQT_OK ||
          ws_vector(ws, right->precision, right->nvec, bytes, 3, &bufs[3]) != GQT_OK)) {
       cudaGetLastError();

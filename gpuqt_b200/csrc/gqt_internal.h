@@ -160,6 +160,7 @@ struct gqt_ham {
   // pattern its length and packed offsets, and its hoppings), per site its record
   // (potential and pattern, 16 bytes), and the launch geometry.
   gqt::StripLattice strip;
+  int strip_loops = 0;  // the loops that run in strips: bit 0 direct, bit 1 symmetric
   int strip_pad = 0;
   int strip_patterns = 0;
   int* strip_pat = nullptr;

@@ -499,6 +499,50 @@ bool split_offset(long long d, long long n, long long d1, int& c0, int& c1)
   return best <= kMaxReach;
 }
 
+// Time of a step of the step loop, us (a symmetric set's gives two moments), on rows of z:
+// it depends on the sites alone. B200, coded operator, at these numbers of sites; beyond the
+// last in proportion.
+double step_loop_us(int n, int z, bool pair)
+{
+  constexpr int kPoints = 8;
+  static const double kSites[kPoints] = {20e3, 65e3, 160e3, 450e3, 1.05e6, 1.35e6, 2.1e6, 4e6};
+  static const double kTime[2][3][kPoints] = {
+    // direct, rows of 3, 4 and 6
+    {{2.18, 2.75, 3.95, 6.3, 11.4, 14.4, 28.0, 53.5},
+     {2.20, 2.83, 3.85, 6.4, 11.6, 14.3, 28.1, 51.1},
+     {2.20, 2.72, 3.95, 7.3, 14.5, 19.5, 36.6, 65.6}},
+    // symmetric
+    {{2.55, 3.25, 4.70, 7.3, 12.7, 15.2, 22.7, 45.0},
+     {2.55, 3.55, 4.70, 7.8, 13.3, 15.9, 24.6, 49.4},
+     {2.55, 3.28, 4.60, 8.4, 15.5, 18.8, 34.4, 64.6}}};
+  const double* t = kTime[pair][z == 3 ? 0 : z == 4 ? 1 : 2];
+  if (n >= kSites[kPoints - 1])
+    return t[kPoints - 1] * n / kSites[kPoints - 1];
+  int k = 1;
+  while (n > kSites[k])
+    ++k;
+  const double f = std::max(0.0, (n - kSites[k - 1]) / (kSites[k] - kSites[k - 1]));
+  return t[k - 1] + f * (t[k] - t[k - 1]);
+}
+
+// The same of the strip loop: iterations times the time of one (steps x columns cells; a
+// lattice of few columns, or one that leaves few of a strip's columns after the halo, takes
+// more of them), and the launch. B200, 927 lattices of 624 to 4 million sites, 10 to 2,000
+// columns, reach 1 to 8, full and short rows, real and complex hoppings: within 10 % but for
+// a few of less than 3,000 sites or 20 columns (20 %).
+double strip_loop_us(const StripGeo& g, int n, int z, bool real, bool pad, bool pair)
+{
+  static const double kLine[2][3][4] = {
+    // columns 32, 64, 96, 128; complex hoppings, rows of 3, 4 and 6
+    {{0.68, 0.94, 1.10, 1.10}, {0.68, 0.80, 0.92, 0.92}, {0.74, 0.92, 1.02, 1.05}},
+    // real
+    {{0.66, 0.71, 0.77, 0.73}, {0.65, 0.75, 0.80, 0.81}, {0.73, 0.78, 0.95, 0.98}}};
+  const double line = kLine[real][z == 3 ? 0 : z == 4 ? 1 : 2][g.cols / 32 - 1] +
+                      (pad ? 0.05 : 0.0) + (pair ? 0.03 : 0.0);
+  const double launch = 0.5 + (pair ? 1.0 : 0.0) + (n >= 1400000 ? 6.0 : g.cols == 128 ? 1.5 : 0.0);
+  return (launch + line * (g.b1 + 3 * (g.steps - 1))) / g.steps;
+}
+
 }  // namespace
 
 StripLattice strip_lattice(int n, const int* delta, int count, int* packed)
@@ -553,15 +597,13 @@ StripLattice strip_lattice(int n, const int* delta, int count, int* packed)
 //   square 1000 x 1001    11.4 / 6.83   4 of 96: 10.8 / 5.62   3 of 128: 11.2 / 5.70
 //   graphene 2,097,152    28.1 / 13.0   4 of 96: 21.2 / 10.6   3 of 128: 21.1 / 10.0
 //   square 2000 x 2000    51.5 / 25.6   4 of 96: 37.5 / 18.7   3 of 128: 37.1 / 17.5
-StripGeo strip_geometry(const gqt_ham* h)
+StripGeo strip_geometry(const gqt_ham* h, int patterns)
 {
   const StripLattice& L = h->strip;
-  if (!L.d1 || !h->strip_rec || h->n_real > 1)
-    return {};
   static const int kShapes[][2] = {{6, 32}, {6, 64}, {4, 96}, {3, 128}};
   const int first = h->n < 20000 ? 0 : h->n < 300000 ? 1 : h->n < 1400000 ? 2 : 3;
   const int sms = device_info().sms;
-  const size_t tables = table_bytes(h->strip_patterns, h->z, h->real_hop, h->strip_pad);
+  const size_t tables = table_bytes(patterns, h->z, h->real_hop, h->strip_pad);
   for (int k = first; k < 4; ++k) {
     StripGeo g;
     g.steps = kShapes[k][0];
@@ -590,6 +632,25 @@ StripGeo strip_geometry(const gqt_ham* h)
   return {};
 }
 
+// The loops that run in strips, bit 0 the direct one, bit 1 the symmetric one: those whose
+// strips are expected to take no longer than the step loop, give or take the 2.5 % at which as
+// many lattices are decided wrongly one way as the other. Of the 927 lattices, direct and
+// symmetric, 10 run 3 to 11 % slower so than step by step (none slower than the step loop was
+// before programmatic launches), and for 7 a gain of 5 to 13 % is left. Without the
+// comparison, us a step in strips / step by step: thin lattices 184 / 28 (square 210,000 x
+// 10), 39 / 7.8 (60,000 x 10); slabs 24.2 / 14.7 (cubic 420 x 420 x 6); long reaches 16.3 /
+// 11.1 (rows of four, 6 columns, 1000 x 1001); graphene with complex hoppings 18.8 / 14.5
+// (600 x 580).
+int strip_loops(const gqt_ham* h, const StripGeo& g)
+{
+  int loops = 0;
+  for (int pair = 0; g.steps && pair < 2; ++pair)
+    if (strip_loop_us(g, h->n, h->z, h->real_hop, h->strip_pad, pair) <=
+        1.025 * step_loop_us(h->n, h->z, pair))
+      loops |= 1 << pair;
+  return loops;
+}
+
 gqt_status strip_upload(gqt_ham* h, const RowPatterns& rp)
 {
   const int z = h->z, np = (int)rp.len.size();
@@ -600,6 +661,10 @@ gqt_status strip_upload(gqt_ham* h, const RowPatterns& rp)
   if (!h->strip.d1)
     return GQT_OK;
   h->strip_pad = h->uniform ? 0 : 1;
+  const StripGeo geo = strip_geometry(h, np);
+  h->strip_loops = strip_loops(h, geo);
+  if (!h->strip_loops)
+    return GQT_OK;
   std::vector<int> pat((size_t)np * (z + 1));
   for (int k = 0; k < np; ++k) {
     pat[(size_t)k * (z + 1)] = rp.len[k];
@@ -633,7 +698,7 @@ gqt_status strip_upload(gqt_ham* h, const RowPatterns& rp)
   }
   cudaFree(pid);
   GQT_CUDA(e);
-  h->strip_geo = strip_geometry(h);
+  h->strip_geo = geo;
   return GQT_OK;
 }
 

@@ -119,3 +119,54 @@ def test_strip_loop_does_not_depend_on_the_set_length():
     for M in range(1, 17):
         got = g.moments(H, phi, phi, M)
         assert np.array_equal(got[0], long[0][:M]) and np.array_equal(got[1], long[1][:M])
+
+
+def slab(n0, n1, n2):
+    """Cubic n0 x n1 x n2, periodic: lines of n1 * n2 sites, a reach of n2 columns."""
+    n = n0 * n1 * n2
+    i = np.arange(n)
+    z, y, x = i % n2, i // n2 % n1, i // (n1 * n2)
+    at = lambda a, b, c: ((a % n0) * n1 + b % n1) * n2 + c % n2  # noqa: E731
+    nl = np.stack([at(x + 1, y, z), at(x - 1, y, z), at(x, y + 1, z), at(x, y - 1, z),
+                   at(x, y, z + 1), at(x, y, z - 1)], 1)
+    return dict(n=n, max_neighbor=6, energy_max=9.0, neighbor_number=np.full(n, 6),
+                neighbor_list=nl.reshape(-1), potential=np.cos(1.7 * i),
+                hopping_real=np.full(6 * n, -1.0), hopping_imag=np.zeros(6 * n))
+
+
+ROUTES = [
+    # the operator; whether the direct and the symmetric loop run in strips
+    (lambda: lattice(SQUARE, 250, 260), True, True),
+    (lambda: lattice(SQUARE, 6500, 10), False, False),      # 10 of a strip's 64 columns
+    (lambda: lattice(GRAPHENE, 7000, 3), False, False),
+    (lambda: lattice(FAR, 60, 61), True, True),
+    (lambda: slab(64, 65, 2), True, True),
+    (lambda: slab(64, 64, 6), False, False),                # half of the columns are halo
+    (lambda: lattice(SQUARE, 500, 500, flux=False, pbc=(False, True)), True, True),
+    (lambda: lattice(GRAPHENE, 300, 300, flux=True), False, False),  # complex, rows of three
+    (lambda: lattice(SQUARE, 99, 90, flux=True), True, True),
+]
+
+
+@pytest.mark.parametrize("case", range(len(ROUTES)))
+def test_strips_only_where_they_are_faster(case):
+    make, direct, sym = ROUTES[case]
+    ell = make()
+    H = g.Hamiltonian(**ell)
+    assert H.format == g.FORMAT_CODED
+    n, M = ell["n"], 41
+    ph = np.random.default_rng(case).uniform(0, 2 * np.pi, n)
+    phi = g.Vector.from_host(np.cos(ph), np.sin(ph))
+    calls = (lambda: g.moments(H, phi, phi, M), lambda: g.moments_doubled(H, phi, M))
+
+    def run(call):
+        g.reset_launch_count()
+        mu = call()
+        return mu[0] + 1j * mu[1], g.launch_count()
+
+    got = [run(c) for c in calls]
+    H.set_format(g.FORMAT_ELL)
+    for (mu, launches), strips, call in zip(got, (direct, sym), calls):
+        want, steps = run(call)
+        assert (launches < steps) == strips and (strips or launches == steps)
+        np.testing.assert_allclose(mu, want, rtol=0, atol=1e-15 * n)

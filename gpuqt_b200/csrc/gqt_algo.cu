@@ -148,7 +148,9 @@ Op make_op(const gqt_ham* h, int nvec = 1)
   op.pot_r = h->pot_r;
   op.xx = h->xx;
   op_emax(op, h->energy_max);
-  if (h->use_codes && h->n_real == 1 && h->stage_nw > 0 && h->stage_err) {
+  if (h->no_code_pack) {
+    // no memory for the packed codes: the unstaged step
+  } else if (h->use_codes && h->n_real == 1 && h->stage_nw > 0 && h->stage_err) {
     op.stage_nw = h->stage_nw;
     op.stage_stages = h->stage_stages;
     for (int w = 0; w < h->stage_nw; ++w) {
@@ -893,8 +895,7 @@ extern "C" gqt_status gqt_vec_segment_sum(const gqt_vec* in, int segment, int co
 
 // ------------------------------------------------------------------ moments
 static gqt_status moments_prepare(const gqt_ham* h, const gqt_vec* left, const gqt_vec* right,
-                                  int M, bool pair, const FormOps** f, void* (&bufs)[4],
-                                  DotScratch** ds)
+                                  int M, const FormOps** f, void* (&bufs)[4], DotScratch** ds)
 {
   const char* w = "gqt_moments";
   GQT_TRY(check_pair(h, right, w));
@@ -913,14 +914,6 @@ static gqt_status moments_prepare(const gqt_ham* h, const gqt_vec* left, const g
     const size_t bytes = right->bytes;
     GQT_TRY(ws_vector(ws, right->precision, right->nvec, bytes, 0, &bufs[0]));
     GQT_TRY(ws_vector(ws, right->precision, right->nvec, bytes, 1, &bufs[1]));
-    // The strip loop writes its vectors beside the two it reads: two more buffers. A
-    // lattice that leaves no memory for them runs step by step.
-    if (strip_eligible(h, right, pair) &&
-        (ws_vector(ws, right->precision, right->nvec, bytes, 2, &bufs[2]) != GQT_OK ||
-         ws_vector(ws, right->precision, right->nvec, bytes, 3, &bufs[3]) != GQT_OK)) {
-      cudaGetLastError();
-      bufs[2] = bufs[3] = nullptr;
-    }
   }
   // Block partials: [grid][R][V][4] doubles for a batch, [grid][V][4] otherwise, followed
   // by the slab of a window of deferred moments.
@@ -930,6 +923,43 @@ static gqt_status moments_prepare(const gqt_ham* h, const gqt_vec* left, const g
   return GQT_OK;
 }
 
+// Whether `bytes` of device memory that a faster loop could do without may be taken: a small
+// amount, or one that leaves nearly all of the free memory to the program.
+static bool may_take(size_t bytes)
+{
+  if (bytes <= (size_t)256 << 20)
+    return true;
+  size_t left = 0, total = 0;
+  return cudaMemGetInfo(&left, &total) == cudaSuccess && bytes <= left / 8;
+}
+
+// What a set of M moments in strips needs beyond the step loop: the sites' records and two
+// more vectors (the launches write beside the two vectors they read). bufs[2] stays null,
+// and the set runs step by step, where no step would run in strips (another loop, too few
+// moments) or the memory is short.
+static void strip_prepare(const gqt_ham* h, const gqt_vec* right, int M, bool pair,
+                          void* (&bufs)[4])
+{
+  if (!strip_eligible(h, right, pair) || (pair ? M / 2 : M - 1) < 2 ||
+      (wave_eligible(h, right, pair) && h->wave_halo >= 0))
+    return;
+  Workspace& ws = *h->ws;
+  std::vector<void*>& held = ws.bufs[{right->precision, right->nvec}].v;
+  const size_t had = held.size();
+  const size_t more = had < 4 ? 4 - had : 0;
+  if (!may_take(more * right->bytes + (h->strip_rec ? 0 : (size_t)h->n * sizeof(uint4))))
+    return;
+  if (strip_records(h) == GQT_OK &&
+      ws_vector(ws, right->precision, right->nvec, right->bytes, 3, &bufs[3]) == GQT_OK) {
+    bufs[2] = held[2];
+    return;
+  }
+  cudaGetLastError();
+  for (; held.size() > had; held.pop_back())
+    cudaFree(held.back());
+  bufs[3] = nullptr;
+}
+
 // The moment loop (direct, or the symmetric pair loop) as one CUDA graph launch.
 static gqt_status moments_run(const gqt_ham* h, const gqt_vec* left, const gqt_vec* right,
                               int M, void* mu_dev, bool pair, const char* w)
@@ -937,7 +967,7 @@ static gqt_status moments_run(const gqt_ham* h, const gqt_vec* left, const gqt_v
   const FormOps* f;
   void* bufs[4] = {nullptr, nullptr, nullptr, nullptr};
   DotScratch* ds;
-  GQT_TRY(moments_prepare(h, left, right, M, pair, &f, bufs, &ds));
+  GQT_TRY(moments_prepare(h, left, right, M, &f, bufs, &ds));
   if (!mu_dev)
     return fail(GQT_ERR_ARG, "%s: null output", w);
   Workspace& ws = *h->ws;
@@ -984,6 +1014,15 @@ static gqt_status moments_run(const gqt_ham* h, const gqt_vec* left, const gqt_v
       GQT_CUDA(cudaStreamCreateWithFlags(&ws.capture_stream, cudaStreamNonBlocking));
       GQT_CUDA(cudaEventCreateWithFlags(&ws.ev_in, cudaEventDisableTiming));
       GQT_CUDA(cudaEventCreateWithFlags(&ws.ev_out, cudaEventDisableTiming));
+    }
+    strip_prepare(h, right, M, pair, bufs);
+    if (const int dot = pair ? kDotPair : kDotLeft;
+        (right->precision == GQT_FP32 || right->precision == GQT_FP32R) &&
+        stage_plan(make_op(h, right->nvec), right->nvec, dot, right->precision == GQT_FP32R,
+                   nullptr, h->n_real) > 0) {
+      const gqt_status st = ensure_code_pack(h);
+      if (st != GQT_OK && h->n_real > 1)  // (a batch has no unstaged FP32R step)
+        return st;
     }
     cudaStream_t saved = s;
     gqt_set_stream(ws.capture_stream);

@@ -130,6 +130,9 @@ gqt_status stage_step(const Op& op, int nvec, int mode, int dot, const void* t0,
 int stage_plan(const Op& op, int nvec, int dot, bool f32, int* windows, int R = 1);
 // The FP32R form's split potential of h (gqt_ham::pot_r), made on first use.
 gqt_status ensure_pot_r(const gqt_ham* h);
+// Packs the codes of h for the staged step unless they are; on failure h is left without
+// (gqt_ham::no_code_pack).
+gqt_status ensure_code_pack(const gqt_ham* h);
 // Grid size for a grid-stride kernel: enough blocks to cover `total` elements, capped
 // at the number of blocks that are resident at once on all SMs.
 int grid_for(const void* kernel, size_t total);

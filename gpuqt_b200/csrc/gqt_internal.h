@@ -111,7 +111,10 @@ struct gqt_ham {
   // most GQT_MAX_CODES distinct values, as lattice models do): one byte per entry and
   // a small table holding the same doubles, so results are unchanged.
   uint8_t* code = nullptr;      // [z*n] column-major
-  void* code_pack = nullptr;    // rows of 3, 4 or 6: each site's z codes, 4 or 8 bytes
+  // rows of 3, 4 or 6: each site's z codes, 4 or 8 bytes, made on the staged step's first use;
+  // no_code_pack: the memory for them was short, and one model's step runs unstaged
+  mutable void* code_pack = nullptr;
+  mutable bool no_code_pack = false;
   int real_hop = 0;             // every hopping of the table is real
   int* code_delta = nullptr;    // [n_codes]: j - i
   double2* code_hop = nullptr;  // [n_codes]
@@ -157,15 +160,17 @@ struct gqt_ham {
   int* stage_rtab = nullptr;
   // Strip moment loop of the FP64 form (gqt_strip.cu): the coded operator as a lattice of
   // lines, whether some rows are short, the distinct rows (per
-  // pattern its length and packed offsets, and its hoppings), per site its record
-  // (potential and pattern, 16 bytes), and the launch geometry.
+  // pattern its length and packed offsets, and its hoppings), per site its pattern and, from
+  // the loop's first use, instead its record (potential and pattern, 16 bytes), and the
+  // launch geometry.
   gqt::StripLattice strip;
   int strip_loops = 0;  // the loops that run in strips: bit 0 direct, bit 1 symmetric
   int strip_pad = 0;
   int strip_patterns = 0;
   int* strip_pat = nullptr;
   double2* strip_hop = nullptr;
-  uint4* strip_rec = nullptr;
+  mutable uint8_t* strip_site = nullptr;
+  mutable uint4* strip_rec = nullptr;
   gqt::StripGeo strip_geo;
   std::unique_ptr<gqt::Workspace> ws;
   ~gqt_ham();

@@ -447,6 +447,7 @@ gqt_ham::~gqt_ham()
   cudaFree(stage_rtab);
   cudaFree(strip_pat);
   cudaFree(strip_hop);
+  cudaFree(strip_site);
   cudaFree(strip_rec);
 }
 
@@ -974,19 +975,6 @@ gqt_status upload_packed(const Packed& P, double energy_max, bool has_xx, gqt_ha
     for (const double2& t : chop)
       if (t.y != 0.0)
         h->real_hop = 0;
-    if (P.z == 3 || P.z == 4 || P.z == 6) {
-      const size_t word = P.z <= 4 ? sizeof(unsigned) : sizeof(uint2);
-      GQT_CUDA(cudaMalloc(&h->code_pack, (size_t)P.n * word));
-      const int grid = std::min((P.n + kBlock - 1) / kBlock, max_grid());
-      GQT_TRY(uploads_done());
-      if (P.z <= 4)
-        k_pack_codes<<<grid, kBlock, 0, stream()>>>(h->code, P.n, P.z, (unsigned*)h->code_pack);
-      else
-        k_pack_codes<<<grid, kBlock, 0, stream()>>>(h->code, P.n, P.z, (uint2*)h->code_pack);
-      count_launches(1);
-      GQT_CUDA(cudaGetLastError());
-      GQT_CUDA(cudaStreamSynchronize(stream()));
-    }
     if (batch_offset)
       GQT_TRY(plan_stage_windows_batch(P, codes, delta, *batch_offset, *batch_n, h));
     else {

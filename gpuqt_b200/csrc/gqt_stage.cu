@@ -998,7 +998,7 @@ gqt_status staged_v(const Op& op, int mode, int dot, const StageLayout& sl, cons
 static bool stage_fits(const Op& op, int nvec, int mode, int dot, bool f32, StageLayout& sl,
                        int R = 1)
 {
-  if (op.stage_nw <= 0 || !op.code_pack || !op.stage_err || (mode != kApply && mode != kCheb))
+  if (op.stage_nw <= 0 || !op.code || !op.stage_err || (mode != kApply && mode != kCheb))
     return false;
   if ((op.stage_rtab != nullptr) != (R > 1) || (R > 1 && !f32))
     return false;
@@ -1121,6 +1121,28 @@ gqt_status ensure_pot_r(const gqt_ham* h)
   const int grid = (h->n + kBlock - 1) / kBlock < max_grid() ? (h->n + kBlock - 1) / kBlock
                                                              : max_grid();
   k_split_pot<<<grid, kBlock, 0, stream()>>>(h->pot, 1.0 / h->energy_max, h->pot_r, h->n);
+  count_launches(1);
+  GQT_CUDA(cudaGetLastError());
+  return GQT_OK;
+}
+
+gqt_status ensure_code_pack(const gqt_ham* h)
+{
+  if (h->code_pack)
+    return GQT_OK;
+  const size_t word = h->z <= 4 ? sizeof(unsigned) : sizeof(uint2);
+  const cudaError_t e = cudaMalloc(&h->code_pack, (size_t)h->n * word);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    h->code_pack = nullptr;
+    h->no_code_pack = true;
+    return cuda_fail(e, "packed codes of the staged step", __FILE__, __LINE__);
+  }
+  const int grid = std::min((h->n + kBlock - 1) / kBlock, max_grid());
+  if (h->z <= 4)
+    k_pack_codes<<<grid, kBlock, 0, stream()>>>(h->code, h->n, h->z, (unsigned*)h->code_pack);
+  else
+    k_pack_codes<<<grid, kBlock, 0, stream()>>>(h->code, h->n, h->z, (uint2*)h->code_pack);
   count_launches(1);
   GQT_CUDA(cudaGetLastError());
   return GQT_OK;

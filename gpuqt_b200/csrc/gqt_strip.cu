@@ -672,33 +672,34 @@ gqt_status strip_upload(gqt_ham* h, const RowPatterns& rp)
       pat[(size_t)k * (z + 1) + 1 + m] = packed[(size_t)k * z + m];
   }
   h->strip_patterns = np;
-  uint8_t* pid = nullptr;
   GQT_CUDA(cudaMalloc(&h->strip_pat, pat.size() * sizeof(int)));
   GQT_CUDA(cudaMemcpy(h->strip_pat, pat.data(), pat.size() * sizeof(int), cudaMemcpyHostToDevice));
   GQT_CUDA(cudaMalloc(&h->strip_hop, rp.hop.size() * sizeof(double2)));
   GQT_CUDA(cudaMemcpy(h->strip_hop, rp.hop.data(), rp.hop.size() * sizeof(double2),
                       cudaMemcpyHostToDevice));
-  // A lattice that leaves no memory for the records runs step by step.
-  if (cudaMalloc(&h->strip_rec, (size_t)h->n * sizeof(uint4)) != cudaSuccess ||
-      cudaMalloc(&pid, (size_t)h->n) != cudaSuccess) {
-    cudaGetLastError();
-    cudaFree(h->strip_rec);
-    h->strip_rec = nullptr;
-    return GQT_OK;
-  }
-  cudaError_t e = cudaMemcpy(pid, rp.site.data(), (size_t)h->n, cudaMemcpyHostToDevice);
-  // (pageable memory, legacy stream: the copies may still be on their way)
-  if (e == cudaSuccess)
-    e = cudaStreamSynchronize(cudaStreamLegacy);
-  if (e == cudaSuccess) {
-    const int grid = std::min((h->n + kBlock - 1) / kBlock, max_grid());
-    k_strip_rec<<<grid, kBlock, 0, stream()>>>(h->pot, pid, h->n, h->strip_rec);
-    count_launches(1);
-    e = cudaStreamSynchronize(stream());
-  }
-  cudaFree(pid);
-  GQT_CUDA(e);
+  GQT_CUDA(cudaMalloc(&h->strip_site, (size_t)h->n));
+  GQT_CUDA(cudaMemcpy(h->strip_site, rp.site.data(), (size_t)h->n, cudaMemcpyHostToDevice));
   h->strip_geo = geo;
+  return GQT_OK;
+}
+
+gqt_status strip_records(const gqt_ham* h)
+{
+  if (h->strip_rec)
+    return GQT_OK;
+  uint4* rec = nullptr;
+  GQT_CUDA(cudaMalloc(&rec, (size_t)h->n * sizeof(uint4)));
+  const int grid = std::min((h->n + kBlock - 1) / kBlock, max_grid());
+  k_strip_rec<<<grid, kBlock, 0, stream()>>>(h->pot, h->strip_site, h->n, rec);
+  count_launches(1);
+  const cudaError_t e = cudaStreamSynchronize(stream());
+  if (e != cudaSuccess) {
+    cudaFree(rec);
+    return cuda_fail(e, "records of the strip loop", __FILE__, __LINE__);
+  }
+  h->strip_rec = rec;
+  cudaFree(h->strip_site);
+  h->strip_site = nullptr;
   return GQT_OK;
 }
 

@@ -23,6 +23,9 @@ struct RowPatterns {
 // Fills h's strip_* members (at upload).
 gqt_status strip_upload(gqt_ham* h, const RowPatterns& rp);
 
+// Makes h's records unless they are made (before a capture: it allocates).
+gqt_status strip_records(const gqt_ham* h);
+
 // `levels` (at most strip_geo.steps) steps of the FP64 loop on one vector: reads T_{k-2}
 // (p2), T_{k-1} (p1) and, unless pair, left; writes the last step's vector to o1 and, if
 // levels >= 2, the one before it to o2, which are none of the inputs. Step m's block

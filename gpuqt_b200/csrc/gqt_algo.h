@@ -11,10 +11,11 @@
 namespace gqt {
 
 struct Workspace {
-  // Temporary vectors per (precision, nvec), allocated on first use and reused.
+  // Temporary vectors per (precision, nvec), allocated two at a time on first use and reused.
   struct Bufs {
     size_t bytes = 0;
     std::vector<void*> v;
+    std::vector<void*> owned;  // the allocations they lie in
   };
   std::map<std::pair<int, int>, Bufs> bufs;
   double2* acc = nullptr;  // FP64 accumulator of the FP32 form's evolution

@@ -161,15 +161,15 @@ struct gqt_ham {
   // Strip moment loop of the FP64 form (gqt_strip.cu): the coded operator as a lattice of
   // lines, whether some rows are short, the distinct rows (per
   // pattern its length and packed offsets, and its hoppings), per site its pattern and, from
-  // the loop's first use, instead its record (potential and pattern, 16 bytes), and the
-  // launch geometry.
+  // the loop's first use, its record (potential and pattern, 16 bytes), and the launch
+  // geometry.
   gqt::StripLattice strip;
   int strip_loops = 0;  // the loops that run in strips: bit 0 direct, bit 1 symmetric
   int strip_pad = 0;
   int strip_patterns = 0;
   int* strip_pat = nullptr;
   double2* strip_hop = nullptr;
-  mutable uint8_t* strip_site = nullptr;
+  uint8_t* strip_site = nullptr;
   mutable uint4* strip_rec = nullptr;
   gqt::StripGeo strip_geo;
   std::unique_ptr<gqt::Workspace> ws;

@@ -8,6 +8,7 @@
 #include <atomic>
 #include <mutex>
 #include <thread>
+#include <new>
 #include <unordered_map>
 #include <vector>
 
@@ -438,16 +439,11 @@ gqt_ham::~gqt_ham()
   cudaFree(pot);
   cudaFree(pot_r);
   cudaFree(tile_first_all);  // tile_first points into it
-  cudaFree(code);
+  cudaFree(code_hop);  // code, code_delta and code_xx point into it
   cudaFree(code_pack);
-  cudaFree(code_delta);
-  cudaFree(code_hop);
-  cudaFree(code_xx);
   cudaFree(stage_err);
   cudaFree(stage_rtab);
-  cudaFree(strip_pat);
-  cudaFree(strip_hop);
-  cudaFree(strip_site);
+  cudaFree(strip_hop);  // strip_pat and strip_site point into it
   cudaFree(strip_rec);
 }
 
@@ -617,24 +613,25 @@ bool build_codes(const Packed& P, std::vector<uint8_t>& codes, std::vector<int>&
   // Pass 1: per column and chunk of rows, the keys in first-seen order; merged in the
   // order of a serial scan (column by column, rows ascending), the codes number the
   // distinct entries by first appearance whatever the chunking.
+  // (One call for all columns: starting 16 threads takes some 0.3 ms.)
   std::atomic<bool> overflow{false};
   Dict dict;
-  for (int m = 0; m < P.z && !overflow; ++m) {
-    std::vector<std::vector<Key>> firsts(17);
-    parallel_rows(P.n, [&](long long lo, long long hi, int chunk) {
+  std::vector<std::vector<Key>> firsts((size_t)P.z * 16);
+  parallel_rows(P.n, [&](long long lo, long long hi, int chunk) {
+    for (int m = 0; m < P.z && !overflow; ++m) {
       Dict local;
       for (long long i = lo; i < hi; ++i)
         if (local.add(key_at(m, i)) < 0) {
           overflow = true;
           return;
         }
-      firsts[chunk] = std::move(local.keys);
-    });
-    for (auto& f : firsts)
-      for (const Key& k : f)
-        if (!overflow && dict.add(k) < 0)
-          overflow = true;
-  }
+      firsts[(size_t)m * 16 + chunk] = std::move(local.keys);
+    }
+  });
+  for (auto& f : firsts)
+    for (const Key& k : f)
+      if (!overflow && dict.add(k) < 0)
+        overflow = true;
   if (overflow)
     return false;
   for (const Key& k : dict.keys) {
@@ -663,97 +660,123 @@ bool build_codes(const Packed& P, std::vector<uint8_t>& codes, std::vector<int>&
   return true;
 }
 
-// The last few keys met, with their values: neighbouring sites alternate among the orbitals
-// of a cell.
-struct RecentKeys {
-  uint64_t key[8];
-  int val[8];
-  int used = 0, next = 0;
-  int find(uint64_t k) const
+// The distinct rows a chunk of sites meets (length and codes), numbered as they come; the last
+// few met first, as neighbouring sites alternate among the orbitals of a cell.
+struct RowDict {
+  uint64_t key[256];
+  int slot[512];  // open addressing, -1 free
+  int count = 0;
+  uint64_t recent[8];
+  int recent_id[8];
+  int recents = 0, next = 0;
+  RowDict() { std::fill(slot, slot + 512, -1); }
+  // the row's number; -1 for a 257th row
+  int add(uint64_t k)
   {
-    for (int i = 0; i < used; ++i)
-      if (key[i] == k)
-        return val[i];
-    return -1;
-  }
-  void add(uint64_t k, int v)
-  {
-    key[next] = k;
-    val[next] = v;
+    for (int i = 0; i < recents; ++i)
+      if (recent[i] == k)
+        return recent_id[i];
+    int s = (int)((k ^ k >> 31) * 0x9e3779b97f4a7c15ull >> 55);
+    while (slot[s] >= 0 && key[slot[s]] != k)
+      s = (s + 1) & 511;
+    if (slot[s] < 0) {
+      if (count == 256)
+        return -1;
+      key[count] = k;
+      slot[s] = count++;
+    }
+    recent[next] = k;
+    recent_id[next] = slot[s];
     next = (next + 1) & 7;
-    used = used < 8 ? used + 1 : 8;
+    recents = recents < 8 ? recents + 1 : 8;
+    return slot[s];
   }
 };
 
-// The distinct rows (length and codes) of a coded operator, at most 256, for the strip
-// moment loop; false when there are more, or its rows are not of 3, 4 or 6 entries.
-bool build_patterns(const Packed& P, const std::vector<uint8_t>& codes,
-                    const std::vector<int>& delta, const std::vector<double2>& hop,
-                    RowPatterns& rp)
+// The distinct rows of a coded operator with rows of at most 7 entries; false when there are
+// more than 256. One pass over the sites: each chunk of them numbers the rows that are new to it
+// after those of a sample, which has nearly all, and where a chunk's numbers differ from the
+// first ones' its sites are renumbered. (Two passes with a hash map took 1.5 ms of an upload of
+// 189,028 sites.)
+bool build_patterns(const Packed& P, const std::vector<uint8_t>& codes, RowPatterns& rp)
 {
-  if (P.z != 3 && P.z != 4 && P.z != 6)
-    return false;
-  // (an operator whose offsets are not lines' needs no patterns)
-  std::vector<int> scratch(delta.size());
-  if (!strip_lattice(P.n, delta.data(), (int)delta.size(), scratch.data()).d1)
-    return false;
+  rp.site.resize(P.n);
   auto key_at = [&](long long i) {
     uint64_t k = (uint64_t)(P.uniform ? P.z : P.nn[i]);
     for (int m = 0; m < P.z; ++m)
       k = k << 8 | codes[(size_t)m * P.n + i];
     return k;
   };
-  // each chunk of rows collects its keys; sorted, they number the patterns
-  std::vector<std::vector<uint64_t>> found(17);
+  RowDict sample;
+  for (long long from : {0LL, (long long)P.n / 2, (long long)P.n - 2048})
+    for (long long i = std::max(0LL, from); i < std::min<long long>(P.n, from + 2048); ++i)
+      if (sample.add(key_at(i)) < 0)
+        return false;
+  std::vector<RowDict> dict(16, sample);
   std::atomic<bool> overflow{false};
   parallel_rows(P.n, [&](long long lo, long long hi, int chunk) {
-    std::unordered_map<uint64_t, int> seen;
-    RecentKeys recent;
-    for (long long i = lo; i < hi && !overflow; ++i) {
-      const uint64_t k = key_at(i);
-      if (recent.find(k) >= 0)
-        continue;
-      recent.add(k, 0);
-      if (seen.emplace(k, 0).second && seen.size() > 256)
-        overflow = true;
-    }
-    for (const auto& kv : seen)
-      found[chunk].push_back(kv.first);
-  });
-  if (overflow)
-    return false;
-  std::vector<uint64_t> keys;
-  for (const auto& f : found)
-    keys.insert(keys.end(), f.begin(), f.end());
-  std::sort(keys.begin(), keys.end());
-  keys.erase(std::unique(keys.begin(), keys.end()), keys.end());
-  if (keys.size() > 256)
-    return false;
-  for (uint64_t k : keys) {
-    rp.len.push_back((int)(k >> (8 * P.z)));
-    for (int m = 0; m < P.z; ++m) {
-      const int c = (int)(k >> (8 * (P.z - 1 - m)) & 255);
-      rp.delta.push_back(delta[c]);
-      rp.hop.push_back(hop[c]);
-    }
-  }
-  rp.site.resize(P.n);
-  parallel_rows(P.n, [&](long long lo, long long hi, int) {
-    std::unordered_map<uint64_t, int> id;
-    for (size_t k = 0; k < keys.size(); ++k)
-      id[keys[k]] = (int)k;
-    RecentKeys recent;
+    RowDict& d = dict[chunk];
     for (long long i = lo; i < hi; ++i) {
-      const uint64_t k = key_at(i);
-      int at = recent.find(k);
-      if (at < 0) {
-        at = id[k];
-        recent.add(k, at);
+      const int at = d.add(key_at(i));
+      if (at < 0 || overflow) {
+        overflow = true;
+        return;
       }
       rp.site[i] = (uint8_t)at;
     }
   });
+  if (overflow)
+    return false;
+  RowDict all = dict[0];
+  std::vector<std::vector<uint8_t>> to(dict.size());  // empty: the chunk's numbers stand
+  bool renumber = false;
+  for (size_t c = 1; c < dict.size(); ++c) {
+    std::vector<uint8_t> map(dict[c].count);
+    bool same = true;
+    for (int k = 0; k < dict[c].count; ++k) {
+      const int at = all.add(dict[c].key[k]);
+      if (at < 0)
+        return false;
+      map[k] = (uint8_t)at;
+      same = same && at == k;
+    }
+    if (!same)
+      to[c] = std::move(map);
+    renumber = renumber || !same;
+  }
+  if (renumber)
+    parallel_rows(P.n, [&](long long lo, long long hi, int chunk) {
+      if (!to[chunk].empty())
+        for (long long i = lo; i < hi; ++i)
+          rp.site[i] = to[chunk][rp.site[i]];
+    });
+  for (int k = 0; k < all.count; ++k) {
+    rp.len.push_back((int)(all.key[k] >> (8 * P.z)));
+    for (int m = 0; m < P.z; ++m)
+      rp.code.push_back((uint8_t)(all.key[k] >> (8 * (P.z - 1 - m))));
+  }
   return true;
+}
+
+// The strip loop of a coded operator, where one of its loops may run in strips. Memory for the
+// rows' numbers that is short on the host leaves the operator without.
+gqt_status plan_strips(const Packed& P, const std::vector<uint8_t>& codes,
+                       const std::vector<int>& delta, const std::vector<double2>& hop, gqt_ham* h)
+{
+  if (P.z != 3 && P.z != 4 && P.z != 6)
+    return GQT_OK;
+  std::vector<int> packed(delta.size());
+  h->strip = strip_lattice(P.n, delta.data(), (int)delta.size(), packed.data());
+  if (!h->strip.d1 || !strip_possible(h))
+    return GQT_OK;
+  RowPatterns rp;
+  try {
+    if (!build_patterns(P, codes, rp))
+      return GQT_OK;
+  } catch (const std::bad_alloc&) {
+    return GQT_OK;
+  }
+  return strip_upload(h, rp, packed, hop);
 }
 
 // H = H^+ for the packed operator: for every pair of sites, the hoppings of the
@@ -961,14 +984,21 @@ gqt_status upload_packed(const Packed& P, double energy_max, bool has_xx, gqt_ha
   std::vector<double> cxx;
   if (build_codes(P, codes, delta, chop, cxx)) {
     const size_t nc = delta.size();
-    GQT_CUDA(cudaMalloc(&h->code, pairs));
-    GQT_CUDA(cudaMalloc(&h->code_delta, nc * sizeof(int)));
-    GQT_CUDA(cudaMalloc(&h->code_hop, nc * sizeof(double2)));
-    GQT_CUDA(cudaMalloc(&h->code_xx, nc * sizeof(double)));
+    // one allocation and two copies: the table's hoppings, xx and offsets, then the codes
+    const size_t at_xx = nc * sizeof(double2), at_delta = at_xx + nc * sizeof(double),
+                 at_code = (at_delta + nc * sizeof(int) + 255) / 256 * 256;
+    std::vector<unsigned char> table(at_code);
+    std::memcpy(table.data(), chop.data(), at_xx);
+    std::memcpy(table.data() + at_xx, cxx.data(), nc * sizeof(double));
+    std::memcpy(table.data() + at_delta, delta.data(), nc * sizeof(int));
+    unsigned char* dev = nullptr;
+    GQT_CUDA(cudaMalloc(&dev, at_code + pairs));
+    h->code_hop = reinterpret_cast<double2*>(dev);
+    h->code_xx = reinterpret_cast<double*>(dev + at_xx);
+    h->code_delta = reinterpret_cast<int*>(dev + at_delta);
+    h->code = dev + at_code;
+    GQT_CUDA(cudaMemcpy(dev, table.data(), at_code, cudaMemcpyHostToDevice));
     GQT_CUDA(cudaMemcpy(h->code, codes.data(), pairs, cudaMemcpyHostToDevice));
-    GQT_CUDA(cudaMemcpy(h->code_delta, delta.data(), nc * sizeof(int), cudaMemcpyHostToDevice));
-    GQT_CUDA(cudaMemcpy(h->code_hop, chop.data(), nc * sizeof(double2), cudaMemcpyHostToDevice));
-    GQT_CUDA(cudaMemcpy(h->code_xx, cxx.data(), nc * sizeof(double), cudaMemcpyHostToDevice));
     h->n_codes = (int)nc;
     h->use_codes = 1;
     h->real_hop = 1;
@@ -979,9 +1009,7 @@ gqt_status upload_packed(const Packed& P, double energy_max, bool has_xx, gqt_ha
       GQT_TRY(plan_stage_windows_batch(P, codes, delta, *batch_offset, *batch_n, h));
     else {
       plan_stage_windows(P, codes, delta, h);
-      RowPatterns rp;
-      if (build_patterns(P, codes, delta, chop, rp))
-        GQT_TRY(strip_upload(h, rp));
+      GQT_TRY(plan_strips(P, codes, delta, chop, h));
     }
     GQT_CUDA(cudaMalloc(&h->stage_err, sizeof(unsigned)));
     GQT_CUDA(cudaMemset(h->stage_err, 0, sizeof(unsigned)));

@@ -651,33 +651,44 @@ int strip_loops(const gqt_ham* h, const StripGeo& g)
   return loops;
 }
 
-gqt_status strip_upload(gqt_ham* h, const RowPatterns& rp)
+bool strip_possible(gqt_ham* h)
+{
+  h->strip_pad = h->uniform ? 0 : 1;
+  return strip_loops(h, strip_geometry(h, 1)) != 0;
+}
+
+gqt_status strip_upload(gqt_ham* h, const RowPatterns& rp, const std::vector<int>& packed,
+                        const std::vector<double2>& hop)
 {
   const int z = h->z, np = (int)rp.len.size();
-  if (np == 0)
-    return GQT_OK;
-  std::vector<int> packed(rp.delta.size());
-  h->strip = strip_lattice(h->n, rp.delta.data(), (int)rp.delta.size(), packed.data());
-  if (!h->strip.d1)
-    return GQT_OK;
-  h->strip_pad = h->uniform ? 0 : 1;
   const StripGeo geo = strip_geometry(h, np);
   h->strip_loops = strip_loops(h, geo);
   if (!h->strip_loops)
     return GQT_OK;
-  std::vector<int> pat((size_t)np * (z + 1));
-  for (int k = 0; k < np; ++k) {
-    pat[(size_t)k * (z + 1)] = rp.len[k];
-    for (int m = 0; m < z; ++m)
-      pat[(size_t)k * (z + 1) + 1 + m] = packed[(size_t)k * z + m];
-  }
   h->strip_patterns = np;
-  GQT_CUDA(cudaMalloc(&h->strip_pat, pat.size() * sizeof(int)));
-  GQT_CUDA(cudaMemcpy(h->strip_pat, pat.data(), pat.size() * sizeof(int), cudaMemcpyHostToDevice));
-  GQT_CUDA(cudaMalloc(&h->strip_hop, rp.hop.size() * sizeof(double2)));
-  GQT_CUDA(cudaMemcpy(h->strip_hop, rp.hop.data(), rp.hop.size() * sizeof(double2),
-                      cudaMemcpyHostToDevice));
-  GQT_CUDA(cudaMalloc(&h->strip_site, (size_t)h->n));
+  // one allocation: the patterns' hoppings, their lengths and offsets, the sites' patterns
+  const size_t hops = (size_t)np * z * sizeof(double2), ints = (size_t)np * (z + 1) * sizeof(int);
+  std::vector<unsigned char> table(hops + ints);
+  double2* const th = reinterpret_cast<double2*>(table.data());
+  int* const tp = reinterpret_cast<int*>(table.data() + hops);
+  for (int k = 0; k < np; ++k) {
+    tp[k * (z + 1)] = rp.len[k];
+    for (int m = 0; m < z; ++m) {
+      const int c = rp.code[(size_t)k * z + m];
+      tp[k * (z + 1) + 1 + m] = packed[c];
+      th[k * z + m] = hop[c];
+    }
+  }
+  unsigned char* dev = nullptr;
+  if (cudaMalloc(&dev, table.size() + (size_t)h->n) != cudaSuccess) {
+    cudaGetLastError();  // no memory for them: step by step
+    h->strip_loops = 0;
+    return GQT_OK;
+  }
+  h->strip_hop = reinterpret_cast<double2*>(dev);
+  h->strip_pat = reinterpret_cast<int*>(dev + hops);
+  h->strip_site = dev + table.size();
+  GQT_CUDA(cudaMemcpy(dev, table.data(), table.size(), cudaMemcpyHostToDevice));
   GQT_CUDA(cudaMemcpy(h->strip_site, rp.site.data(), (size_t)h->n, cudaMemcpyHostToDevice));
   h->strip_geo = geo;
   return GQT_OK;
@@ -698,8 +709,6 @@ gqt_status strip_records(const gqt_ham* h)
     return cuda_fail(e, "records of the strip loop", __FILE__, __LINE__);
   }
   h->strip_rec = rec;
-  cudaFree(h->strip_site);
-  h->strip_site = nullptr;
   return GQT_OK;
 }
 

@@ -11,17 +11,20 @@ namespace gqt {
 // (c0 & 255) | (c1 & 255) << 8.
 StripLattice strip_lattice(int n, const int* delta, int count, int* packed);
 
-// The distinct rows of a coded operator: pattern k has len[k] entries, entry m of it the
-// offset delta[k * z + m] and hopping hop[k * z + m]; site i has pattern site[i]. Empty
-// when there are more than 256.
+// The distinct rows of a coded operator: pattern k has len[k] entries, entry m of it of code
+// code[k * z + m]; site i has pattern site[i]. At most 256.
 struct RowPatterns {
-  std::vector<int> len, delta;
-  std::vector<double2> hop;
-  std::vector<uint8_t> site;
+  std::vector<int> len;
+  std::vector<uint8_t> code, site;
 };
 
-// Fills h's strip_* members (at upload).
-gqt_status strip_upload(gqt_ham* h, const RowPatterns& rp);
+// Whether a loop of h, whose strip lattice is set, may run in strips if its rows are few.
+bool strip_possible(gqt_ham* h);
+
+// Fills h's strip_* members but the lattice (at upload); packed and hop: per code its packed
+// offset (strip_lattice) and hopping.
+gqt_status strip_upload(gqt_ham* h, const RowPatterns& rp, const std::vector<int>& packed,
+                        const std::vector<double2>& hop);
 
 // Makes h's records unless they are made (before a capture: it allocates).
 gqt_status strip_records(const gqt_ham* h);

@@ -134,3 +134,53 @@ def test_fp32r_at_size(tmp_path):
     ref = g.moments(H, X64, X64, M)
     assert _dos_err(m, g.moments(H, X32, X32, M, precision=g.FP32R), ref) <= DOS_BOUND
     assert _dos_err(m, g.moments_doubled(H, X32, M, precision=g.FP32R), ref) <= DOS_BOUND
+
+
+def _hermitian_flux(z, n0, n1):
+    """Rows of three (a brick wall), four or six (hops across a line doubled) with phases of
+    period 3 on the hops along a line: complex, Hermitian, coded."""
+    n = n0 * n1
+    i = np.arange(n)
+    x, y = i // n1, i % n1
+    at = lambda a, b: (a % n0) * n1 + b % n1  # noqa: E731
+    phase = np.exp(2j * np.pi / 3 * (x % 3))
+    cols = [(at(x, y + 1), phase), (at(x, y - 1), phase.conj())]
+    one = np.ones(n, complex)
+    if z == 3:
+        cols.append((np.where((x + y) % 2 == 0, at(x + 1, y), at(x - 1, y)), one))
+    else:
+        cols += [(at(x + 1, y), one), (at(x - 1, y), one)] * (1 if z == 4 else 2)
+    hop = np.stack([c[1] for c in cols], 1)
+    return dict(n=n, max_neighbor=z, energy_max=8.5, neighbor_number=np.full(n, z),
+                neighbor_list=np.stack([c[0] for c in cols], 1).reshape(-1),
+                potential=np.cos(0.7 * i), hopping_real=hop.real.reshape(-1),
+                hopping_imag=hop.imag.reshape(-1))
+
+
+@pytest.mark.parametrize("z", [3, 4, 6])
+@pytest.mark.parametrize("V", [16, 32])
+def test_fp32r_complex_hoppings_staged_and_in_a_batch(z, V):
+    """The staged step's variant for complex hoppings against the unstaged step, and its batch
+    form against the models alone (E_max 8 is a power of two, so the batch's pre-divided
+    operator has the same FP32 parts)."""
+    ells = [dict(_hermitian_flux(z, *s), energy_max=8.0) for s in ((18, 40), (36, 22))]
+    M, alone, states = 60, [], []
+    for k, ell in enumerate(ells):
+        ph = np.random.default_rng(k).uniform(0, 2 * np.pi, (V, ell["n"]))
+        states.append((np.cos(ph), np.sin(ph)))
+        H = g.Hamiltonian(**ell)
+        X = g.Vector.from_host(*states[-1], nvec=V, precision=g.FP32)
+        sets = lambda: [g.moments(H, X, X, M, precision=g.FP32R)] + (  # noqa: E731
+            [g.moments_doubled(H, X, M, precision=g.FP32R)] if V <= 16 else [])
+        assert H.stage_plan(V, g.FP32R)[0] >= 2
+        staged = sets()
+        H.set_staging(-1)
+        for a, b in zip(staged, sets()):
+            assert _rel(a, b) <= REL
+        alone.append(staged)
+    B = g.Hamiltonian.batch(ells)
+    X = g.Vector.from_host(*B.scatter(states), nvec=V, precision=g.FP32)
+    for j, mu in enumerate([g.moments(B, X, X, M, precision=g.FP32R)] + (
+            [g.moments_doubled(B, X, M, precision=g.FP32R)] if V <= 16 else [])):
+        for r in range(len(ells)):
+            assert _rel((mu[0][r], mu[1][r]), alone[r][j]) <= REL

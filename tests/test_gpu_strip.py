@@ -170,3 +170,68 @@ def test_strips_only_where_they_are_faster(case):
         want, steps = run(call)
         assert (launches < steps) == strips and (strips or launches == steps)
         np.testing.assert_allclose(mu, want, rtol=0, atol=1e-15 * n)
+
+
+# rows of six with a Hermitian flux along the lines (doubled hops across them: a reach of 1)
+SIX = [[(1, 0, 0), (-1, 0, 0), (0, 1, 0), (0, -1, 0), (0, 1, 0), (0, -1, 0)]]
+ROWS = [(hops, n0, n1, pbc, flux)
+        for hops, n0, n1 in ((GRAPHENE, 30, 29), (SQUARE, 48, 61), (SIX, 36, 45))
+        for pbc in ((True, True), (True, False)) for flux in (False, True)]
+
+
+@pytest.mark.parametrize("case", range(len(ROWS)))
+def test_every_kind_of_row_in_both_loops(case):
+    """Rows of 3, 4 and 6, full and short, real and complex, direct and symmetric: the 24
+    kernels."""
+    hops, n0, n1, pbc, flux = ROWS[case]
+    ell = lattice(hops, n0, n1, pbc=pbc, flux=flux, emax=9.9)
+    H = g.Hamiltonian(**ell)
+    n, M = ell["n"], 40
+    ph = np.random.default_rng(case).uniform(0, 2 * np.pi, n)
+    phi = g.Vector.from_host(np.cos(ph), np.sin(ph))
+    left = g.Vector.from_host(np.sin(3 * ph), np.cos(5 * ph))
+    e = np.zeros(n)
+    e[n // 2 + 1] = 1.0
+    unit = g.Vector.from_host(e, np.zeros(n))
+    calls = (lambda: g.moments(H, left, phi, M), lambda: g.moments_doubled(H, phi, M),
+             lambda: g.moments(H, unit, phi, M))
+
+    def run(call):
+        g.reset_launch_count()
+        mu = call()
+        return mu[0] + 1j * mu[1], g.launch_count()
+
+    strips = [run(c) for c in calls]
+    H.set_format(g.FORMAT_ELL)
+    steps = [run(c) for c in calls]
+    for (mu, launches), (want, count) in zip(strips, steps):
+        assert launches < count
+        np.testing.assert_allclose(mu, want, rtol=0, atol=1e-15 * n)
+    assert np.array_equal(strips[2][0], steps[2][0])  # elements of T_k, bit for bit
+
+
+def test_the_largest_shape_element_by_element():
+    """Above 1.4 million sites a launch takes 3 steps of 128 columns: elements of T_k at a
+    strip's and a segment's edges, odd numbers of lines and columns."""
+    n0, n1 = 1201, 1203
+    ell = lattice(SQUARE, n0, n1)
+    H = g.Hamiltonian(**ell)
+    n, M = ell["n"], 20
+    ph = np.random.default_rng(0).uniform(0, 2 * np.pi, n)
+    phi = g.Vector.from_host(np.cos(ph), np.sin(ph))
+    sites = [0, n - 1, n1 - 1, n // 2, *(k * n1 + j for k in (56, 57, 58, 600)
+                                         for j in (110, 120, 121, 241))]
+    units = []
+    for s in sites:
+        e = np.zeros(n)
+        e[s] = 1.0
+        units.append(g.Vector.from_host(e, np.zeros(n)))
+    g.reset_launch_count()
+    got = [g.moments(H, e, phi, M) for e in units]
+    launches = g.launch_count()
+    H.set_format(g.FORMAT_ELL)
+    g.reset_launch_count()
+    want = [g.moments(H, e, phi, M) for e in units]
+    assert launches < g.launch_count()
+    for a, w in zip(got, want):
+        assert np.array_equal(a[0], w[0]) and np.array_equal(a[1], w[1])

@@ -272,6 +272,13 @@ __device__ __forceinline__ int code_of(uint2 w, int m)
   return ((m < 4 ? w.x : w.y) >> (8 * (m & 3))) & 255;
 }
 
+// Bytes of a code's hopping in the form's table (more than 32 would leave a batch of several
+// models and many codes, its stages at their largest, no room that it had).
+__host__ __device__ constexpr int stage_hop_bytes(bool f32)
+{
+  return f32 ? 2 * (int)sizeof(float4) : (int)sizeof(double2);
+}
+
 // MULTI: one step of a realisation batch (op.stage_rtab: each model's windows; md: the
 // models' tiles and the per-block, per-model sum slots that k_tile_reduce combines).
 // Tiles never straddle two models (every model is padded to 1024 sites). A block's
@@ -297,15 +304,18 @@ __global__ void __launch_bounds__(kStageThreads, 2)
   // per stage: full (the copies have landed) and empty (every compute warp has read it)
   uint64_t* full = reinterpret_cast<uint64_t*>(stage_smem + (size_t)S * sl.stage_bytes);
   uint64_t* empty = full + kMaxStages;
+  // the table of hoppings of the form: GQT_FP32 the FP64 ones; GQT_FP32R those divided by
+  // E_max as FP32 (hi, lo) parts, each twice: (hi.x, hi.x, lo.x, lo.x), then (-hi.y, hi.y,
+  // -lo.y, lo.y)
   double2* hop = reinterpret_cast<double2*>(empty + kMaxStages);
-  // GQT_FP32R: the hoppings divided by E_max as FP32 (hi, lo) parts, each twice: (hi.x,
-  // hi.x, lo.x, lo.x), then (-hi.y, hi.y, -lo.y, lo.y)
-  float4* hopf = reinterpret_cast<float4*>(hop + op.n_codes);
+  float4* hopf = reinterpret_cast<float4*>(hop);
+  unsigned char* const tables =
+    reinterpret_cast<unsigned char*>(hop) + op.n_codes * stage_hop_bytes(F32);
   // per code: byte offset in a stage of site 0's neighbour row (-1: gathered from global
   // memory), and the offset j - i. MULTI: the byte offsets per model and code (coff) and
   // the offsets j - i per code (cdelta) instead.
-  int2* cinfo = reinterpret_cast<int2*>(hopf + 2 * op.n_codes);
-  int* coff = reinterpret_cast<int*>(hopf + 2 * op.n_codes);
+  int2* cinfo = reinterpret_cast<int2*>(tables);
+  int* coff = reinterpret_cast<int*>(tables);
   // MULTI: md's fields as values (lambdas then capture no kernel parameter by address)
   const int R = MULTI ? md.n_real : 1;
   const int* const tile_first = md.tile_first;
@@ -318,10 +328,13 @@ __global__ void __launch_bounds__(kStageThreads, 2)
   __shared__ int abort_flag;  // MULTI: a wait ran out; the block computes no further
 
   for (int c = threadIdx.x; c < op.n_codes; c += blockDim.x) {
-    hop[c] = op.code_hop[c];
-    const float4 hf = scaled_hop(op.code_hop[c], op);
-    hopf[2 * c] = make_float4(hf.x, hf.x, hf.z, hf.z);
-    hopf[2 * c + 1] = make_float4(-hf.y, hf.y, -hf.w, hf.w);
+    if constexpr (F32) {
+      const float4 hf = scaled_hop(op.code_hop[c], op);
+      hopf[2 * c] = make_float4(hf.x, hf.x, hf.z, hf.z);
+      hopf[2 * c + 1] = make_float4(-hf.y, hf.y, -hf.w, hf.w);
+    } else {
+      hop[c] = op.code_hop[c];
+    }
     if constexpr (!MULTI) {
       const int d = op.code_delta[c];
       int o = -1;
@@ -878,13 +891,13 @@ bool stage_layout(const Op& op, int V, int mode, int dot, int stages, StageLayou
   return false;
 }
 
-// Dynamic shared memory of a launch beside its stages: the barriers, the hopping table in
-// FP64 and FP32 parts and the code offsets (R > 1, a realisation batch of R models: per
-// model and code, with the offsets j - i per code and each model's window starts).
-size_t stage_table_bytes(const Op& op, int R)
+// Dynamic shared memory of a launch beside its stages: the barriers, the form's hopping table
+// and the code offsets (R > 1, a realisation batch of R models: per model and code, with the
+// offsets j - i per code and each model's window starts).
+size_t stage_table_bytes(const Op& op, int R, bool f32)
 {
-  const size_t base = 2 * kMaxStages * sizeof(uint64_t) +
-                      (size_t)op.n_codes * (sizeof(double2) + 2 * sizeof(float4));
+  const size_t base =
+    2 * kMaxStages * sizeof(uint64_t) + (size_t)op.n_codes * stage_hop_bytes(f32);
   if (R <= 1)
     return base + (size_t)op.n_codes * sizeof(int2);
   return base + ((size_t)R * op.n_codes + op.n_codes + (size_t)R * (kStageWin + 1)) * sizeof(int);
@@ -899,7 +912,7 @@ size_t stage_table_bytes(const Op& op, int R)
 int multi_stage_budget(const Op& op, int R, int V, int dot)
 {
   const int kVS = dot == kDotPair ? 2 * V : V;
-  const int added = (int)stage_table_bytes(op, R) - (int)stage_table_bytes(op, 1);
+  const int added = (int)stage_table_bytes(op, R, true) - (int)stage_table_bytes(op, 1, true);
   return (104 << 10) - added - kComputeWarps * kVS * 4 * (int)sizeof(double);
 }
 
@@ -910,7 +923,7 @@ gqt_status launch_staged_as(const Op& op, const StageLayout& sl, const float2* t
 {
   auto* kernel = k_step_staged<V, Z, MODE, DOT, F32, MULTI, REAL>;
   const int R = MULTI ? md.n_real : 1;
-  const size_t smem = (size_t)sl.stages * sl.stage_bytes + stage_table_bytes(op, R);
+  const size_t smem = (size_t)sl.stages * sl.stage_bytes + stage_table_bytes(op, R, F32);
   static std::mutex mu;
   static std::unordered_map<size_t, int> per_sm;  // blocks per SM by shared memory size
   static size_t attr = 0;                         // the kernel's shared memory limit set

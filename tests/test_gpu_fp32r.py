@@ -184,3 +184,38 @@ def test_fp32r_complex_hoppings_staged_and_in_a_batch(z, V):
             [g.moments_doubled(B, X, M, precision=g.FP32R)] if V <= 16 else [])):
         for r in range(len(ells)):
             assert _rel((mu[0][r], mu[1][r]), alone[r][j]) <= REL
+
+
+def test_fp32r_batch_with_the_largest_stages_and_many_codes():
+    """Eight models, 241 codes, two stages of 100 KB asked for: the tables beside the stages
+    leave about 1 KB of a block's shared memory. Offsets 0 to 336 in one window (32 sites of 32
+    vectors a tile); short rows at the end of each model; not Hermitian."""
+    n, z, V, M = 2016, 6, 32, 12
+    offsets = np.unique(np.round(np.linspace(0, 336, 241)).astype(int))[1:]
+    assert len(offsets) == 240
+    i = np.arange(n)
+    pick = offsets[(i % 40)[:, None] + 40 * np.arange(z)[None, :]]
+    order = np.argsort(i[:, None] + pick >= n, axis=1, kind="stable")
+    to = np.take_along_axis(i[:, None] + pick, order, 1)
+    inside = to < n
+    ells, states, alone = [], [], []
+    for k in range(8):
+        ells.append(dict(n=n, max_neighbor=z, energy_max=8.0, neighbor_number=inside.sum(1),
+                         neighbor_list=np.where(inside, to, i[:, None]).reshape(-1),
+                         potential=np.cos((k + 1) * i),
+                         hopping_real=np.where(inside, -1.0, 0.0).reshape(-1),
+                         hopping_imag=np.zeros(n * z)))
+        ph = np.random.default_rng(k).uniform(0, 2 * np.pi, (V, n))
+        states.append((np.cos(ph), np.sin(ph)))
+        H = g.Hamiltonian(**ells[-1])
+        H.set_staging(-1)
+        x = g.Vector.from_host(*states[-1], nvec=V, precision=g.FP32)
+        alone.append(g.moments(H, x, x, M, precision=g.FP32R))
+    B = g.Hamiltonian.batch(ells)
+    assert B.n_codes == 241
+    B.set_staging(2)
+    assert B.stage_plan(V, g.FP32R) == (2, 1)
+    X = g.Vector.from_host(*B.scatter(states), nvec=V, precision=g.FP32)
+    mu = g.moments(B, X, X, M, precision=g.FP32R)
+    for r in range(8):
+        assert _rel((mu[0][r], mu[1][r]), alone[r]) <= REL

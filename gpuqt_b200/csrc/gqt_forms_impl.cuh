@@ -80,6 +80,24 @@ gqt_status launch_op_pdl(void (*kernel)(Op, KArgs...), size_t total, const Op& o
                     op, args...);
 }
 
+// The same where the launch has at most `per_sm` blocks for an SM, and plain above. The unstaged
+// FP32, FP32X and FP32R steps gain from the overlap only while the launches themselves count:
+// the early blocks of a larger step crowd on the SMs that end first, and take other lines than
+// the step before left in those SMs' half of L2. B200, us per step plain / overlapped: FP32 16
+// vectors on 3,480 sites 4.72 / 4.32, 14,640 5.93 / 6.16, 52,800 9.33 / 9.65, 160,800 17.02 /
+// 17.37; 32 vectors on 9,000 sites 6.99 / 7.68; FP32X 16 vectors on 3,480 sites 6.04 / 5.60,
+// 52,800 13.2 / 13.7; FP32R 4 vectors on 14,640 sites 4.88 / 4.33, 65,536 6.53 / 7.16
+// (symmetric 4.44 / 5.07), 1,046,528 symmetric 16.4 / 17.6. FP32 4 vectors gain up to four
+// blocks for an SM: 52,800 sites 6.32 / 5.74, 160,800 9.40 / 9.17, 361,200 12.9 / 13.3.
+template <typename... KArgs, typename... Args>
+gqt_status launch_op_pdl_upto(int per_sm, void (*kernel)(Op, KArgs...), size_t total, const Op& op,
+                              Args... args)
+{
+  const bool overlap = total <= (size_t)per_sm * device_info().sms * kBlock;
+  return launch_pdl(kernel, grid_for((const void*)kernel, total), kBlock, op_smem_bytes(op),
+                    overlap, op, args...);
+}
+
 template <typename K, typename... Args>
 gqt_status launch_smem(K* kernel, size_t total, size_t smem, Args... args)
 {
@@ -143,16 +161,20 @@ struct OpImpl {
         auto run = [&](auto wc) -> gqt_status {
           constexpr int WW = decltype(wc)::value;
           const size_t items = (size_t)op.n * (V / WW);
+          // (FP64: any number of blocks)
+          constexpr int kPerSm =
+            !Fp32Like<VT2>::value ? 1 << 20 : std::is_same<VT2, float2>::value && V == 4 ? 4 : 1;
+          auto launch = [&](auto* kernel) -> gqt_status {
+            return launch_op_pdl_upto(kPerSm, kernel, items, op, a0, a1, o, l, d);
+          };
           if (mode == kApply) {
             if (dot)
-              return launch_op_pdl(k_step_vec<VT2, V, WW, Z, A, kApply, true, C>, items, op, a0, a1, o, l,
-                            d);
-            return launch_op_pdl(k_step_vec<VT2, V, WW, Z, A, kApply, false, C>, items, op, a0, a1, o, l,
-                          d);
+              return launch(k_step_vec<VT2, V, WW, Z, A, kApply, true, C>);
+            return launch(k_step_vec<VT2, V, WW, Z, A, kApply, false, C>);
           }
           if (dot)
-            return launch_op_pdl(k_step_vec<VT2, V, WW, Z, A, kCheb, true, C>, items, op, a0, a1, o, l, d);
-          return launch_op_pdl(k_step_vec<VT2, V, WW, Z, A, kCheb, false, C>, items, op, a0, a1, o, l, d);
+            return launch(k_step_vec<VT2, V, WW, Z, A, kCheb, true, C>);
+          return launch(k_step_vec<VT2, V, WW, Z, A, kCheb, false, C>);
         };
         if constexpr (W2 != W) {
           if (op.wpt == W2)
@@ -200,11 +222,13 @@ struct OpImpl {
         constexpr int Z = decltype(zc)::value;
         if constexpr (V > 1) {
           const size_t items = (size_t)op.n * (V / WP);
+          // (FP32 4 vectors, 641,600 sites 10.8 / 10.4 us, 1,001,000 sites 15.8 / 16.5)
+          constexpr int kPerSm = std::is_same<VT2, float2>::value ? 18 : 1 << 20;
           if (mode == kApply)
-            return launch_op_pdl(k_step_vec<VT2, V, WP, Z, A, kApply, kDotPair, C>, items, op, a0,
-                             a1, o, (const VT2*)nullptr, d);
-          return launch_op_pdl(k_step_vec<VT2, V, WP, Z, A, kCheb, kDotPair, C>, items, op, a0, a1,
-                           o, (const VT2*)nullptr, d);
+            return launch_op_pdl_upto(kPerSm, k_step_vec<VT2, V, WP, Z, A, kApply, kDotPair, C>,
+                                      items, op, a0, a1, o, (const VT2*)nullptr, d);
+          return launch_op_pdl_upto(kPerSm, k_step_vec<VT2, V, WP, Z, A, kCheb, kDotPair, C>, items,
+                                    op, a0, a1, o, (const VT2*)nullptr, d);
         } else {
           const size_t total = (size_t)op.n * V;
           if (mode == kApply)

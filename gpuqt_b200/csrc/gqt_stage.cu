@@ -1269,8 +1269,8 @@ gqt_status run_r(const Op& op, int mode, const void* t0, const void* t1, void* o
   return with_z(op.z, [&](auto zc) -> gqt_status {
     constexpr int Z = decltype(zc)::value;
     if (mode == kApply)
-      return launch_op_pdl(k_step_r<V, Z, kApply, DOT, C>, items, op, a0, a1, o, lf, d);
-    return launch_op_pdl(k_step_r<V, Z, kCheb, DOT, C>, items, op, a0, a1, o, lf, d);
+      return launch_op_pdl_upto(1, k_step_r<V, Z, kApply, DOT, C>, items, op, a0, a1, o, lf, d);
+    return launch_op_pdl_upto(1, k_step_r<V, Z, kCheb, DOT, C>, items, op, a0, a1, o, lf, d);
   });
 }
 

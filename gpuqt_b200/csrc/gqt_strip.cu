@@ -36,6 +36,8 @@ namespace {
 
 constexpr int kStripThreads = 384;  // most computing threads of a block: steps x columns
 constexpr int kStripBlocks = 2;     // blocks per SM (72 registers a thread)
+// Most dynamic shared memory of a block, with which two fit an SM.
+constexpr size_t kStripSmem = (113 << 10) - 2048;
 // Lines of a vector ring: an iteration reads lines q - 2 .. q + 1 of a step's ring and
 // writes q + 2; input line q replaces q - 6, whose last reader is iteration q - 5, and is
 // copied from then on, two iterations before its first reader.
@@ -616,7 +618,7 @@ StripGeo strip_geometry(const gqt_ham* h, int patterns)
     g.b0 = (L.d1 + g.strips - 1) / g.strips;
     g.smem = (size_t)((g.steps + 1) * kRing + rec_ring(g.steps)) * g.cols * 16 + 2 * kGuard +
              tables;
-    if (2 * (g.smem + 2048) > (size_t)226 << 10)
+    if (g.smem > kStripSmem)
       continue;
     // one wave of two blocks per SM
     const int segs = std::min(L.lines, sms * kStripBlocks / g.strips);
@@ -736,8 +738,10 @@ gqt_status strip_steps(const gqt_ham* h, const Op& op, bool pair, int levels, co
   sa.stride = stride;
   sa.counter = counter;
   auto go = [&](auto* kernel) -> gqt_status {
+    // (the same limit for every lattice: one of its own would take the room from a larger
+    // lattice's launch that another thread is about to make)
     GQT_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                  (int)geo.smem));
+                                  (int)kStripSmem));
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(geo.grid);
     cfg.blockDim = dim3(geo.steps * geo.cols + 32);

@@ -235,3 +235,45 @@ def test_the_largest_shape_element_by_element():
     assert launches < g.launch_count()
     for a, w in zip(got, want):
         assert np.array_equal(a[0], w[0]) and np.array_equal(a[1], w[1])
+
+
+def test_lattices_of_several_shapes_side_by_side():
+    """Lattices whose launches take different amounts of shared memory share a kernel: replayed
+    in turn, and captured at the same time by threads, each gives its own moments."""
+    import threading
+
+    def model(k, n0, n1):
+        H = g.Hamiltonian(**lattice(SQUARE, n0, n1, seed=k))
+        ph = np.random.default_rng(k).uniform(0, 2 * np.pi, H.n)
+        return H, g.Vector.from_host(np.cos(ph), np.sin(ph))
+
+    sizes = ((40, 44), (250, 260), (640, 700))  # 6 steps of 32 and of 64 columns, 4 of 96
+    models = [model(k, *s) for k, s in enumerate(sizes)]
+    lengths = range(20, 60)
+    want = [[g.moments(H, x, x, M) for M in lengths] for H, x in models]
+    for M in (20, 33):
+        for _ in range(2):
+            for (H, x), w in zip(models, want):
+                got = g.moments(H, x, x, M)
+                assert np.array_equal(got[0], w[M - 20][0])
+                assert np.array_equal(got[1], w[M - 20][1])
+    bad = []
+
+    def work(k):
+        try:
+            for _ in range(2):
+                H, x = model(k, *sizes[k])  # nothing captured yet
+                for M, w in zip(lengths, want[k]):
+                    got = g.moments(H, x, x, M)
+                    if not (np.array_equal(got[0], w[0]) and np.array_equal(got[1], w[1])):
+                        bad.append((k, M))
+                H.close()
+        except Exception as e:  # reported by the assertion below
+            bad.append((k, repr(e)))
+
+    threads = [threading.Thread(target=work, args=(k,)) for k in range(3)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not bad, bad[:3]

@@ -14,8 +14,8 @@ Also reported, on the same line:
   forms         graphene 2M in every form: FP64 on the ELL arrays, FP32 storage with
                 1/16/32 vectors per launch, symmetric (doubled) sets in FP64 and FP32,
                 each with its byte model and roofline fraction; `target_ratios` states the
-                FP32/FP64 ratios like for like (direct/direct, doubled/doubled) next to
-                their byte-model ceilings
+                FP32/FP64 ratios like for like (direct/direct, doubled/doubled), next to
+                their byte-model ceilings where the FP64 loop is HBM-bound
   evolution     the Bessel evolution of one 1 fs MSD step (evolve, evolvex)
   batch         the realisation batch (8 uneven square lattices, 64 vectors, FP32)
   cubic256      the 3D Anderson lattice 256^3 (z = 6): FP64 and 16-vector FP32 side by
@@ -62,16 +62,28 @@ def entry_bytes(coded):
     return 1 if coded else 4 + 16
 
 
-# The FP64 loop on the coded operator of this lattice runs in strips, STRIP_STEPS steps
-# per launch: a launch reads T_{m-1}, T_{m-2}, left and a 16-byte record per site (potential
-# and row pattern) and writes the last two vectors.
-STRIP_STEPS = 3
-
-
-def fp64_bytes_per_site(z=Z, coded=True):
-    if coded:
-        return (5 * 16 + 16) / STRIP_STEPS
+# Where the FP64 loop runs in strips, `steps` Chebyshev steps per launch (1: step by step), a
+# launch reads T_{m-1}, T_{m-2}, left and a 16-byte record per site (potential and row
+# pattern) and writes the last two vectors.
+def fp64_bytes_per_site(z=Z, coded=True, steps=1):
+    if steps > 1:
+        return (5 * 16 + 16) / steps
     return z * entry_bytes(coded) + 8 + 4 * 16
+
+
+def steps_per_launch(g, H, x, symmetric=False):
+    """Chebyshev steps per launch of the FP64 moment loop on H, from launch counts: 120 steps
+    more take 120 / steps launches more (and one that combines their partial sums)."""
+    def launches(steps):
+        g.reset_launch_count()
+        if symmetric:
+            g.moments_doubled(H, x, 2 * (steps + 1))
+        else:
+            g.moments(H, x, x, steps + 2)
+        return g.launch_count()
+
+    launches(120)  # what the first set prepares is launched once
+    return round(120 / (launches(120) - launches(0) - 1))
 
 
 def fp32_bytes_per_site_vector(V, z=Z, coded=True):
@@ -86,9 +98,9 @@ def fp32x_bytes_per_site_vector(V, z=Z, coded=True):
 
 # A step of a symmetric (doubled) moment set reads T_{k-1} and T_{k-2} and writes T_k
 # (no left stream) and yields two moments.
-def fp64_pair_bytes_per_site_step(z=Z, coded=True):
-    if coded:
-        return (4 * 16 + 16) / STRIP_STEPS
+def fp64_pair_bytes_per_site_step(z=Z, coded=True, steps=1):
+    if steps > 1:
+        return (4 * 16 + 16) / steps
     return z * entry_bytes(coded) + 8 + 3 * 16
 
 
@@ -393,6 +405,8 @@ def run_ours(args):
         x = g.Vector.from_host(*phi)
         mu = torch.empty(2 * M, dtype=torch.float64, device="cuda")
 
+        per = steps_per_launch(g, H, x)
+
         # --- plain FP64 moment sets, inputs resident in HBM
         for _ in range(args.warmup):
             g.moments_device(H, x, x, M, mu.data_ptr())
@@ -415,16 +429,16 @@ def run_ours(args):
         value = world * n * M * args.steps / (ms / 1e3)
         coded = H.format == g.FORMAT_CODED
         fmt = "coded" if coded else "ell"
-        per = STRIP_STEPS if coded else 1  # Chebyshev steps per launch
         per_launch_s = t0.elapsed_time(t1) / 1e3 / (args.steps * M) * per
-        bpl = fp64_bytes_per_site(coded=coded) * n * per
+        bpl = fp64_bytes_per_site(coded=coded, steps=per) * n * per
         achieved = bpl / per_launch_s / 1e9
         traffic = None
         tp = os.path.join(ROOT, "profiles", "traffic.json")
         if os.path.exists(tp):
             with open(tp) as f:
                 traffic = json.load(f).get(
-                    ("k_strip_fp64" if coded else "k_step_fp64_ell") +
+                    ("k_strip_fp64" if per > 1 else "k_step_fp64_coded" if coded else
+                     "k_step_fp64_ell") +
                     "_graphene2m_bytes_per_launch")
 
         # --- e2e: host phase vector (pinned) -> device, moments -> host, every step
@@ -495,8 +509,8 @@ def run_ours(args):
                 "roofline": {"bound": "hbm", "achieved": achieved, "peak": hbm_peak,
                              "unit": "GB/s", "frac": achieved / hbm_peak,
                              "traffic": traffic, "peak_kind": peak_kind,
-                             "kernel": f"k_strip<Z=3,dot> ({STRIP_STEPS} steps per launch)"
-                             if coded else "k_step<double2,V=1,Z=3,Exact,kCheb,dot> (ell)",
+                             "kernel": f"k_strip<Z=3,dot> ({per} steps per launch)" if per > 1 else
+                             f"k_step<double2,V=1,Z=3,Exact,kCheb,dot> ({fmt})",
                              "bytes_per_launch": bpl},
                 "cpu_baseline": cpu,
                 "e2e": e2e,
@@ -621,8 +635,15 @@ def measure_forms(g, torch, m, H, phi, args, stream, hbm_peak):
     H.set_format(default)
     for k in [k for k in out if k.startswith("fp32")]:
         out[k]["speedup_vs_fp64"] = out[k]["site_moments_per_s"] / rate64
-    out["fp32x_v16"]["byte_ceiling_vs_fp64"] = (fp64_bytes_per_site(coded=coded) /
-                                                fp32x_bytes_per_site_vector(16, coded=coded))
+    # The ratio of two forms' byte models bounds their rates' while both are HBM-bound, which
+    # the FP64 loop in strips is not: no ceiling then.
+    steps, steps2 = steps_per_launch(g, H, x64), steps_per_launch(g, H, x64, symmetric=True)
+
+    def ceiling(fp64_bytes, fp64_steps, other):
+        return fp64_bytes(coded=coded) / other if fp64_steps == 1 else None
+
+    out["fp32x_v16"]["byte_ceiling_vs_fp64"] = ceiling(
+        fp64_bytes_per_site, steps, fp32x_bytes_per_site_vector(16, coded=coded))
     out["fp64_v1_site_moments_per_s"] = rate64
 
     # Symmetric moment sets from half the Chebyshev steps (gqt_moments_doubled): the
@@ -652,7 +673,7 @@ def measure_forms(g, torch, m, H, phi, args, stream, hbm_peak):
          "max_err_vs_direct": float(np.max(np.hypot(dr - r64, di - i64)) /
                                     np.max(np.hypot(r64, i64))),
          "speedup_vs_fp64": rate64_dbl / rate64},
-        **pair_roofline(rate64_dbl, fp64_pair_bytes_per_site_step(coded=coded)))
+        **pair_roofline(rate64_dbl, fp64_pair_bytes_per_site_step(coded=coded, steps=steps2)))
     vecs = [phi] + [m.initial_state() for _ in range(15)]
     X16 = g.Vector.from_host(np.stack([v[0] for v in vecs]), np.stack([v[1] for v in vecs]),
                              nvec=16, precision=g.FP32)
@@ -704,18 +725,19 @@ def measure_forms(g, torch, m, H, phi, args, stream, hbm_peak):
     out["fp64_v1_ell"] = {"site_moments_per_s": rate64_ell, "achieved_gbs": ach,
                           "frac": ach / hbm_peak,
                           "bytes_per_site_moment": fp64_bytes_per_site(coded=False)}
-    ach = fp64_bytes_per_site(coded=coded) * rate64 / 1e9
+    b64 = fp64_bytes_per_site(coded=coded, steps=steps)
+    ach = b64 * rate64 / 1e9
     out["fp64_v1"] = {"site_moments_per_s": rate64, "achieved_gbs": ach,
-                      "frac": ach / hbm_peak,
-                      "bytes_per_site_moment": fp64_bytes_per_site(coded=coded)}
+                      "frac": ach / hbm_peak, "bytes_per_site_moment": b64,
+                      "steps_per_launch": steps}
 
     # The target ratio, like for like: batched FP32 storage over plain FP64 in the
-    # same loop (direct over direct, doubled over doubled), each next to the ratio of
-    # the two forms' byte models, which bounds it while both are HBM-bound.
+    # same loop (direct over direct, doubled over doubled).
     d32 = out["fp32_v16"]
-    ceil_direct = fp64_bytes_per_site(coded=coded) / fp32_bytes_per_site_vector(16, coded=coded)
-    ceil_dbl = (fp64_pair_bytes_per_site_step(coded=coded) /
-                fp32_pair_bytes_per_site_vector_step(16, coded=coded))
+    ceil_direct = ceiling(fp64_bytes_per_site, steps,
+                          fp32_bytes_per_site_vector(16, coded=coded))
+    ceil_dbl = ceiling(fp64_pair_bytes_per_site_step, steps2,
+                       fp32_pair_bytes_per_site_vector_step(16, coded=coded))
     ratio_direct = d32["site_moments_per_s"] / rate64
     ratio_dbl = rate32_dbl / rate64_dbl
     out["target_ratios"] = {
@@ -742,10 +764,9 @@ def measure_forms(g, torch, m, H, phi, args, stream, hbm_peak):
                                       out["fp32r_v16_doubled"]["site_moments_per_s"] /
                                       rate64_dbl) >= 3.0 and
                                   d32["frac"] >= 0.7 and out["fp64_v1"]["frac"] >= 0.7),
-        "note": "while both forms are HBM-bound the like-for-like ratio is capped by "
-                "the byte models (byte_ceiling_*): FP32 storage keeps four 8-byte vector "
-                "streams per site-vector-moment (three in a doubled step) against 75 B "
-                "(59 B) for the coded FP64 step"}
+        "note": "byte_ceiling_*: the ratio of the two forms' byte models, a cap on the "
+                "like-for-like ratio while both are HBM-bound; null where the FP64 loop runs "
+                "in strips (bound by instruction issue, not by HBM)"}
     # Bessel evolution of one MSD step (1 fs): evolve and evolvex, FP64.
     dt = m.time_step[0] * m.energy_max
     st = x64.clone()
@@ -810,6 +831,7 @@ def measure_cubic(g, torch, tmp, stream, hbm_peak, vectors=16):
     vecs = [m.initial_state() for _ in range(vectors)]
     x64 = g.Vector.from_host(*vecs[0])
     mu64 = torch.empty(2 * M, dtype=torch.float64, device="cuda")
+    steps = steps_per_launch(g, H, x64)
     ms64 = timed(lambda: g.moments_device(H, x64, x64, M, mu64.data_ptr()))
     r64, i64 = g.moments(H, x64, x64, M)
     X = g.Vector.from_host(np.stack([v[0] for v in vecs]), np.stack([v[1] for v in vecs]),
@@ -820,7 +842,7 @@ def measure_cubic(g, torch, tmp, stream, hbm_peak, vectors=16):
     ms32 = timed(lambda: g.moments_device(H, X, X, M, mu32.data_ptr()))
     mu_h = mu32.view(M, vectors, 2).cpu().numpy()
     dos = P.compare(g, m, (r64, i64), (mu_h[:, 0, 0].copy(), mu_h[:, 0, 1].copy()))
-    b64 = fp64_bytes_per_site(z=z, coded=coded)
+    b64 = fp64_bytes_per_site(z=z, coded=coded, steps=steps)
     b32 = fp32_bytes_per_site_vector(vectors, z=z, coded=coded)
     rate64 = n * M / (ms64 / 1e3)
     rate32 = vectors * n * M / (ms32 / 1e3)
@@ -863,7 +885,7 @@ def measure_cubic(g, torch, tmp, stream, hbm_peak, vectors=16):
         "fp64": form(rate64, ms64, b64, 1, parts["fp64"]),
         "fp32_v16": form(rate32, ms32, b32, vectors, parts["fp32_v16"]),
         "speedup_dos": rate32 / rate64,
-        "byte_ceiling_dos": b64 / b32,
+        "byte_ceiling_dos": b64 / b32 if steps == 1 else None,
         "evolution_fp64": {"dt_scaled": dt, "bessel_terms": terms,
                            "k_cheb2_frac": gb_e / hbm_peak, "k_cheb2_gbs": gb_e,
                            "k_cheb2x_frac": gb_x / hbm_peak, "k_cheb2x_gbs": gb_x},

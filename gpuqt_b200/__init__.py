@@ -392,8 +392,9 @@ class Hamiltonian:
         _call("gqt_ham_set_batch_tile", self.h, int(tile_sites))
 
     def set_loop(self, window: int, chunk_sites: int = 0) -> None:
-        """Moment loop of the FP64 form: 0 one launch per step, S >= 2 the wavefront
-        loop of S steps per launch over chunks of chunk_sites sites (0: 1024)
+        """Moment loop of the FP64 form: 0, the default, in strips (3 to 6 steps per launch)
+        on plane lattices where that is faster, else one launch per step; S >= 2 the
+        wavefront loop, S steps per launch over chunks of chunk_sites sites (0: 1024)
         (gqt_ham_set_loop)."""
         _call("gqt_ham_set_loop", self.h, int(window), int(chunk_sites))
 

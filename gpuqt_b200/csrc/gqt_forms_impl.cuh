@@ -53,7 +53,8 @@ gqt_status launch_op(K* kernel, size_t total, const Op& op, Args... args)
 // next kernel's blocks are scheduled, and have loaded their tables, when the previous
 // kernel's last blocks end. B200, 100 moments, plain / overlapped: 4 FP64 vectors on 2,400
 // sites 377 / 327 us, cubic 20^3 symmetric FP64 183 / 152, FP32 16 vectors on cubic 20^3
-// 563 / 481, FP32R 16 vectors on 1,047,040 sites 8.85 / 8.79 ms.
+// 563 / 481, FP32R 16 vectors on 1,047,040 sites 8.85 / 8.79 ms (where it does not pay:
+// launch_op_pdl_upto).
 template <typename... KArgs, typename... Args>
 gqt_status launch_pdl(void (*kernel)(KArgs...), int grid, int threads, size_t smem, bool pdl,
                       Args... args)

@@ -189,7 +189,8 @@ struct ExactArith {
   // their loops cost every iteration the moves of the calling convention and the
   // constants that cannot stay in registers across it (FP64 moment sets 1-4 % slower).
   // The evolution and current kernels (scale) call it: they live on many resident warps
-  // with few registers, and divide_any inlined made them 1-20 % slower.
+  // with few registers, and divide_any inlined made them 1-20 % slower; so do symmetric
+  // sets on rows of four in k_step_vec.
   static constexpr unsigned kDivLo = 2u * ((1023u - 900u) << 20);
   static constexpr unsigned kDivSpan = 2u * (1800u << 20);
   static __device__ __forceinline__ unsigned div_key(double a)

@@ -82,14 +82,19 @@ gqt_status launch_op_pdl(void (*kernel)(Op, KArgs...), size_t total, const Op& o
 }
 
 // The same where the launch has at most `per_sm` blocks for an SM, and plain above. The unstaged
-// FP32, FP32X and FP32R steps gain from the overlap only while the launches themselves count:
+// FP32, FP32X and FP32R steps, and many-vector FP64 steps on the ELL arrays, gain from the
+// overlap only while the launches themselves count:
 // the early blocks of a larger step crowd on the SMs that end first, and take other lines than
 // the step before left in those SMs' half of L2. B200, us per step plain / overlapped: FP32 16
 // vectors on 3,480 sites 4.72 / 4.32, 14,640 5.93 / 6.16, 52,800 9.33 / 9.65, 160,800 17.02 /
 // 17.37; 32 vectors on 9,000 sites 6.99 / 7.68; FP32X 16 vectors on 3,480 sites 6.04 / 5.60,
 // 52,800 13.2 / 13.7; FP32R 4 vectors on 14,640 sites 4.88 / 4.33, 65,536 6.53 / 7.16
-// (symmetric 4.44 / 5.07), 1,046,528 symmetric 16.4 / 17.6. FP32 4 vectors gain up to four
-// blocks for an SM: 52,800 sites 6.32 / 5.74, 160,800 9.40 / 9.17, 361,200 12.9 / 13.3.
+// (symmetric 4.44 / 5.07), 1,046,528 symmetric 16.4 / 17.6. FP32 4 vectors on the coded
+// operator gain up to four blocks for an SM: 52,800 sites 6.32 / 5.74, 160,800 9.40 / 9.17,
+// 361,200 12.9 / 13.3. ELL arrays: FP64 4 vectors on 72,160 sites 7.99 / 7.62, 262,144 20.2 /
+// 23.9, 16 on 72,160 20.1 / 22.0; FP32 4 vectors on 95,098 sites 7.60 / 8.61; symmetric FP64 4
+// vectors on 160,800 5.92 / 5.68, 262,144 11.3 / 12.1; FP32 4 on 72,160 4.69 / 4.57, 95,098
+// 4.46 / 4.87; FP32X 4 on 14,640 2.93 / 2.88, 52,800 3.89 / 4.21.
 template <typename... KArgs, typename... Args>
 gqt_status launch_op_pdl_upto(int per_sm, void (*kernel)(Op, KArgs...), size_t total, const Op& op,
                               Args... args)
@@ -162,9 +167,9 @@ struct OpImpl {
         auto run = [&](auto wc) -> gqt_status {
           constexpr int WW = decltype(wc)::value;
           const size_t items = (size_t)op.n * (V / WW);
-          // (FP64: any number of blocks)
-          constexpr int kPerSm =
-            !Fp32Like<VT2>::value ? 1 << 20 : std::is_same<VT2, float2>::value && V == 4 ? 4 : 1;
+          constexpr int kPerSm = !Fp32Like<VT2>::value                          ? (C ? 1 << 20 : 10)
+                                 : std::is_same<VT2, float2>::value && V == 4 && C ? 4
+                                                                                   : 1;
           auto launch = [&](auto* kernel) -> gqt_status {
             return launch_op_pdl_upto(kPerSm, kernel, items, op, a0, a1, o, l, d);
           };
@@ -190,7 +195,8 @@ struct OpImpl {
       }
       auto go = [&](auto* kernel) -> gqt_status {
         // (a large FP32 step streams while the next one's early blocks would take its
-        // slots: 1,047,040 sites 2 % slower with the overlap, 720,720 sites 1 % faster)
+        // slots: 1,047,040 sites 2 % slower with the overlap, 720,720 sites 1 % faster;
+        // symmetric sets on 1,001,000 to 1,046,528 sites 2-3 % slower, 361,200 3 % faster)
         const bool overlap = std::is_same<VT2, double2>::value || total <= 900000;
         return launch_pdl(kernel, grid_for((const void*)kernel, total), kBlock, op_smem_bytes(op),
                           overlap, op, a0, a1, o, l, d);
@@ -223,8 +229,10 @@ struct OpImpl {
         constexpr int Z = decltype(zc)::value;
         if constexpr (V > 1) {
           const size_t items = (size_t)op.n * (V / WP);
-          // (FP32 4 vectors, 641,600 sites 10.8 / 10.4 us, 1,001,000 sites 15.8 / 16.5)
-          constexpr int kPerSm = std::is_same<VT2, float2>::value ? 18 : 1 << 20;
+          // (coded, FP32 4 vectors: 641,600 sites 10.8 / 10.4 us, 1,001,000 sites 15.8 / 16.5)
+          constexpr int kPerSm = !Fp32Like<VT2>::value                  ? (C ? 1 << 20 : 18)
+                                 : std::is_same<VT2, float2>::value ? (C ? 18 : 2)
+                                                                    : 1;
           if (mode == kApply)
             return launch_op_pdl_upto(kPerSm, k_step_vec<VT2, V, WP, Z, A, kApply, kDotPair, C>,
                                       items, op, a0, a1, o, (const VT2*)nullptr, d);
@@ -232,11 +240,15 @@ struct OpImpl {
                                     op, a0, a1, o, (const VT2*)nullptr, d);
         } else {
           const size_t total = (size_t)op.n * V;
+          // (as in step)
+          auto go = [&](auto* kernel) -> gqt_status {
+            const bool overlap = std::is_same<VT2, double2>::value || total <= 900000;
+            return launch_pdl(kernel, grid_for((const void*)kernel, total), kBlock,
+                              op_smem_bytes(op), overlap, op, a0, a1, o, (const VT2*)nullptr, d);
+          };
           if (mode == kApply)
-            return launch_op_pdl(k_step<VT2, V, Z, A, kApply, kDotPair, C>, total, op, a0, a1,
-                                   o, (const VT2*)nullptr, d);
-          return launch_op_pdl(k_step<VT2, V, Z, A, kCheb, kDotPair, C>, total, op, a0, a1, o,
-                                 (const VT2*)nullptr, d);
+            return go(k_step<VT2, V, Z, A, kApply, kDotPair, C>);
+          return go(k_step<VT2, V, Z, A, kCheb, kDotPair, C>);
         }
       });
     }

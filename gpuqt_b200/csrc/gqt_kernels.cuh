@@ -1833,8 +1833,18 @@ __device__ __forceinline__ double2 accumulate(double2 o, double b, double tr, do
 
 // gpu_chebyshev_2 (src/hamiltonian.cu:465-529): s2 = 2 H s1 / E_max - s0 and
 // out += (label) * bessel * s2. s2 may alias s0.
+// Blocks per SM k_cheb2 is compiled for (0: the compiler's choice). The FP32 terms of many
+// vectors on rows of four and six take 32 registers and fill an SM; left to itself the
+// compiler took 36 after the wait for the previous launch came in, six blocks (cubic 64^3, 16
+// vectors, evolve with dt E_max = 10: 1870 us at eight, 2170 at six).
+template <typename VT2, int V, int Z, bool C>
+constexpr int cheb2_min_blocks()
+{
+  return std::is_same<VT2, float2>::value && C && V >= 4 && (Z == 4 || Z == 6) ? 8 : 0;
+}
+
 template <typename VT2, typename OT2, int V, int Z, class A, bool C>
-__global__ void __launch_bounds__(kBlock) k_cheb2(Op op, const VT2* s0,
+__global__ void __launch_bounds__(kBlock, cheb2_min_blocks<VT2, V, Z, C>()) k_cheb2(Op op, const VT2* s0,
                                                   const VT2* __restrict__ s1, VT2* s2,
                                                   OT2* __restrict__ out, double bessel,
                                                   int label)

@@ -189,8 +189,8 @@ struct ExactArith {
   // their loops cost every iteration the moves of the calling convention and the
   // constants that cannot stay in registers across it (FP64 moment sets 1-4 % slower).
   // The evolution and current kernels (scale) call it: they live on many resident warps
-  // with few registers, and divide_any inlined made them 1-20 % slower; so do symmetric
-  // sets on rows of four in k_step_vec.
+  // with few registers, and divide_any inlined made them 1-20 % slower; so do two kinds of
+  // set in k_step_vec.
   static constexpr unsigned kDivLo = 2u * ((1023u - 900u) << 20);
   static constexpr unsigned kDivSpan = 2u * (1800u << 20);
   static __device__ __forceinline__ unsigned div_key(double a)
@@ -1367,10 +1367,11 @@ __global__ void __launch_bounds__(kBlock, vec_min_blocks<VT2, Z, DOT>()) k_step_
 #pragma unroll
       for (int k = 0; k < W; ++k) {
         const double2 y0 = widen(s.y0[k]);
-        if constexpr (kExact && DOT == kDotPair && Z == 4) {
+        if constexpr (kExact && ((DOT == kDotPair && Z == 4) || (DOT == kDotLeft && Z == 0 && !C))) {
           // (the call is the faster one in symmetric sets on rows of four: 4 and 16 vectors on
-          // 1,001,000 sites 25.6 and 99.7 us, inline 26.6 and 101.7; on rows of three and six
-          // inline is)
+          // 1,001,000 sites 25.6 and 99.7 us, inline 26.6 and 101.7; and in direct sets on ELL
+          // rows of other lengths, where inline code spills: rows of two, 4 and 16 vectors on
+          // 260,000 sites 17.4 and 66.7 us, inline 18.6 and 71.4)
           tr[k] = A::scale(tr[k], op);
           ti[k] = A::scale(ti[k], op);
         } else {

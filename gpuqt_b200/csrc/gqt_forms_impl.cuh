@@ -92,9 +92,9 @@ gqt_status launch_op_pdl(void (*kernel)(Op, KArgs...), size_t total, const Op& o
 // (symmetric 4.44 / 5.07), 1,046,528 symmetric 16.4 / 17.6. FP32 4 vectors on the coded
 // operator gain up to four blocks for an SM: 52,800 sites 6.32 / 5.74, 160,800 9.40 / 9.17,
 // 361,200 12.9 / 13.3. ELL arrays: FP64 4 vectors on 72,160 sites 7.99 / 7.62, 262,144 20.2 /
-// 23.9, 16 on 72,160 20.1 / 22.0; FP32 4 vectors on 95,098 sites 7.60 / 8.61; symmetric FP64 4
-// vectors on 160,800 5.92 / 5.68, 262,144 11.3 / 12.1; FP32 4 on 72,160 4.69 / 4.57, 95,098
-// 4.46 / 4.87; FP32X 4 on 14,640 2.93 / 2.88, 52,800 3.89 / 4.21.
+// 23.9, 16 on 9,000 5.56 / 5.75, 72,160 20.1 / 22.0; FP32 4 vectors on 95,098 sites 7.60 /
+// 8.61; symmetric FP64 4 vectors on 160,800 5.92 / 5.68, 262,144 11.3 / 12.1; FP32 4 on 72,160
+// 4.69 / 4.57, 95,098 4.46 / 4.87; FP32X 4 on 14,640 2.93 / 2.88, 52,800 3.89 / 4.21.
 template <typename... KArgs, typename... Args>
 gqt_status launch_op_pdl_upto(int per_sm, void (*kernel)(Op, KArgs...), size_t total, const Op& op,
                               Args... args)
@@ -167,9 +167,10 @@ struct OpImpl {
         auto run = [&](auto wc) -> gqt_status {
           constexpr int WW = decltype(wc)::value;
           const size_t items = (size_t)op.n * (V / WW);
-          constexpr int kPerSm = !Fp32Like<VT2>::value                          ? (C ? 1 << 20 : 10)
-                                 : std::is_same<VT2, float2>::value && V == 4 && C ? 4
-                                                                                   : 1;
+          // (FP64 on the ELL arrays: 4 vectors up to 10, more never)
+          constexpr bool f64 = !Fp32Like<VT2>::value;
+          constexpr bool f32 = std::is_same<VT2, float2>::value;
+          constexpr int kPerSm = f64 ? (C ? 1 << 20 : V > 4 ? 0 : 10) : f32 && V == 4 && C ? 4 : 1;
           auto launch = [&](auto* kernel) -> gqt_status {
             return launch_op_pdl_upto(kPerSm, kernel, items, op, a0, a1, o, l, d);
           };

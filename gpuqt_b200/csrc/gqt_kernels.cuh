@@ -1367,7 +1367,8 @@ __global__ void __launch_bounds__(kBlock, vec_min_blocks<VT2, Z, DOT>()) k_step_
 #pragma unroll
       for (int k = 0; k < W; ++k) {
         const double2 y0 = widen(s.y0[k]);
-        if constexpr (kExact && ((DOT == kDotPair && Z == 4) || (DOT == kDotLeft && Z == 0 && !C))) {
+        if constexpr (kExact &&
+                      ((DOT == kDotPair && Z == 4) || (DOT == kDotLeft && Z == 0 && !C))) {
           // (the call is the faster one in symmetric sets on rows of four: 4 and 16 vectors on
           // 1,001,000 sites 25.6 and 99.7 us, inline 26.6 and 101.7; and in direct sets on ELL
           // rows of other lengths, where inline code spills: rows of two, 4 and 16 vectors on
